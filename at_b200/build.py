@@ -21,13 +21,16 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + CSRC, "-I" + INCLUDE]
 
+# (object, source, flags); the tracking units are compiled once per kernel
 UNITS = [
-    ("track_exact.cu", ["-fmad=false"]),
-    ("track_fast.cu", ["-fmad=true"]),
-    ("tangent.cu", ["-fmad=false"]),
-    ("adjoint.cu", ["-fmad=false"]),
-    ("atb200.cu", []),
-    ("atb_noalloc.cu", []),
+    *[("track_%s_%s" % (arith, kern.lower()), "track_%s.cu" % arith,
+       ["-fmad=" + fmad, "-DATB_KERNELS=ATB_KERNEL_" + kern])
+      for arith, fmad in (("exact", "false"), ("fast", "true"))
+      for kern in ("BASE", "GEN", "SERVE", "NP2")],
+    ("tangent", "tangent.cu", ["-fmad=false"]),
+    ("adjoint", "adjoint.cu", ["-fmad=false"]),
+    ("atb200", "atb200.cu", []),
+    ("atb_noalloc", "atb_noalloc.cu", []),
 ]
 DEPS = ["atb_physics.cuh", "atb_dual.cuh", "track_kernel.cuh", "tangent_kernel.cuh",
         "adjoint_kernel.cuh",
@@ -54,9 +57,9 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     nv = nvcc()
     deps = [os.path.join(CSRC, d) for d in DEPS] + [os.path.join(INCLUDE, "atb200.h"), __file__]
     objs, jobs = [], []
-    for src, flags in UNITS:
+    for obj, src, flags in UNITS:
         s = os.path.join(CSRC, src)
-        o = os.path.join(BUILD, src.replace(".cu", ".o"))
+        o = os.path.join(BUILD, obj + ".o")
         objs.append(o)
         if force or _stale(o, [s] + deps):
             cmd = [nv, *ARCH, *COMMON, *flags, "-c", s, "-o", o]
@@ -64,7 +67,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
                 cmd += ["-Xptxas", "-v"]
             if verbose:
                 print(" ".join(cmd))
-            jobs.append((src, cmd))
+            jobs.append((obj, cmd))
     # the units are independent: compile them side by side
     running = [(src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.PIPE,
                                       text=True)) for src, cmd in jobs]

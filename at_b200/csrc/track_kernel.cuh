@@ -27,6 +27,20 @@
 #error "define ATB_FAST to 0 or 1"
 #endif
 
+/* the tracking kernels this unit instantiates (each takes a minute to
+   compile, so the build gives each its own unit); the derivative units take
+   none */
+#define ATB_KERNEL_BASE 1
+#define ATB_KERNEL_GEN 2
+#define ATB_KERNEL_SERVE 4
+#define ATB_KERNEL_NP2 8
+#ifdef ATB_NO_TRACK_KERNEL
+#define ATB_KERNELS 0
+#endif
+#ifndef ATB_KERNELS
+#define ATB_KERNELS (ATB_KERNEL_BASE | ATB_KERNEL_GEN | ATB_KERNEL_SERVE | ATB_KERNEL_NP2)
+#endif
+
 #define ATB_CAT2(a, b) a##b
 #define ATB_CAT(a, b) ATB_CAT2(a, b)
 #if ATB_FAST
@@ -786,7 +800,7 @@ __device__ __forceinline__ bool serve_requeue(const AtbServeRing& ring, const At
     return true;
 }
 
-#ifndef ATB_NO_TRACK_KERNEL
+#if ATB_KERNELS
 
 /* lost-particle marking of one particle after an element (pyat/at.c:115-161) */
 __device__ __forceinline__ void apply_loss_rule(const AtbJob& J, P6& r, bool& lost, bool active,
@@ -1310,6 +1324,7 @@ __device__ __forceinline__ void track_tiles(const AtbJob* __restrict__ jobs,
     }
 }
 
+#if ATB_KERNELS & ATB_KERNEL_BASE
 extern "C" __global__ void __launch_bounds__(ATB_MAX_THREADS)
 ATB_CAT(atb_track_kernel, ATB_KSUFFIX)(const AtbJob* __restrict__ jobs,
                                        const AtbTile* __restrict__ tiles, int ntiles,
@@ -1320,7 +1335,9 @@ ATB_CAT(atb_track_kernel, ATB_KSUFFIX)(const AtbJob* __restrict__ jobs,
     track_tiles<1>(jobs, tiles, ntiles, tile_counter, job_next, status, smem_cap_words,
                    scratch);
 }
+#endif
 
+#if ATB_KERNELS & ATB_KERNEL_GEN
 /* with the other integrators of the GPU call (tables with ATB_F_INTEG) */
 extern "C" __global__ void __launch_bounds__(ATB_MAX_THREADS)
 ATB_CAT(ATB_CAT(atb_track_kernel, ATB_KSUFFIX), _gen)(const AtbJob* __restrict__ jobs,
@@ -1333,7 +1350,9 @@ ATB_CAT(ATB_CAT(atb_track_kernel, ATB_KSUFFIX), _gen)(const AtbJob* __restrict__
     track_tiles<1, true>(jobs, tiles, ntiles, tile_counter, job_next, status, smem_cap_words,
                          scratch);
 }
+#endif
 
+#if ATB_KERNELS & ATB_KERNEL_SERVE
 /* The serving loop's persistent kernel: new tiles come from a queue the host
    appends to while it runs (AtbServeCtl), continuations from the device-side
    ring; `done[job]` counts the particles of each job that have run all their
@@ -1347,7 +1366,9 @@ ATB_CAT(atb_serve_kernel, ATB_KSUFFIX)(const AtbJob* __restrict__ jobs,
     track_tiles<1, false, true>(jobs, tiles, 0, tile_counter, nullptr, status, smem_cap_words,
                                 scratch, sv);
 }
+#endif
 
+#if ATB_KERNELS & ATB_KERNEL_NP2
 /* two particles per thread (the autotuner's particles-per-thread choice) */
 extern "C" __global__ void __launch_bounds__(ATB_MAX_THREADS)
 ATB_CAT(ATB_CAT(atb_track_kernel, ATB_KSUFFIX), _np2)(const AtbJob* __restrict__ jobs,
@@ -1360,8 +1381,9 @@ ATB_CAT(ATB_CAT(atb_track_kernel, ATB_KSUFFIX), _np2)(const AtbJob* __restrict__
     track_tiles<2>(jobs, tiles, ntiles, tile_counter, job_next, status, smem_cap_words,
                    scratch);
 }
+#endif
 
-#endif  // ATB_NO_TRACK_KERNEL
+#endif  // ATB_KERNELS
 
 }  // namespace atb
 
