@@ -34,7 +34,7 @@ UNITS = [
 ]
 DEPS = ["atb_physics.cuh", "atb_dual.cuh", "track_kernel.cuh", "tangent_kernel.cuh",
         "adjoint_kernel.cuh",
-        "atb_diffusion.cuh", "atb_integrators.h",
+        "atb_diffusion.cuh", "atb_integrators.h", "atb_rn.h",
         "atb_kernel_api.h", "atb_table.h"]
 
 

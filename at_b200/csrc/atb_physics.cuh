@@ -21,6 +21,7 @@
 
 #include "atb_table.h"
 #include "atb_dual.cuh"
+#include "atb_rn.h"
 
 namespace atb {
 
@@ -192,10 +193,11 @@ __device__ __forceinline__ void horner_fixed(const double* A, const double* B, c
     for (int i = MO - 1; i >= 0; --i) horner_step(re, im, x, y, B[i], A[i]);
 }
 
-/* The same recursion for an upright magnet (every A_n = 0, fast kernels
- * only): the first step starts from Im = 0, so it is re B_MO x + B_{MO-1},
- * im = B_MO y, and later steps add no A_n.  Equal to horner_fixed up to the
- * sign of a zero. */
+/* The same recursion for an upright magnet (every A_n = 0): the first step
+ * starts from Im = 0, so it is re = B_MO x + B_{MO-1}, im = B_MO y, and later
+ * steps add no A_n.  For finite x, y the same values as horner_fixed up to
+ * the sign of a zero (a non-finite coordinate would meet the dropped 0 y as
+ * NaN: the exact kernels send such a magnet through the full recursion). */
 template <int MO, class T>
 __device__ __forceinline__ void horner_upright(const double* B, const T& x, const T& y, T& re,
                                                T& im) {
@@ -203,12 +205,21 @@ __device__ __forceinline__ void horner_upright(const double* B, const T& x, cons
         re = B[0];
         im = 0.0;
     } else {
+#if ATB_FAST
         re = fma(B[MO], x, B[MO - 1]);
+#else
+        re = B[MO] * x + B[MO - 1];
+#endif
         im = B[MO] * y;
 #pragma unroll
         for (int i = MO - 2; i >= 0; --i) {
+#if ATB_FAST
             const T ret = fma(re, x, fma(-im, y, B[i]));
             im = fma(im, x, re * y);
+#else
+            const T ret = re * x - im * y + B[i];
+            im = im * x + re * y;
+#endif
             re = ret;
         }
     }
@@ -391,6 +402,66 @@ __device__ __forceinline__ void diff_drift_pn(P6T<T>& r, double L, const T& pn) 
     r.ct += NormL * p_norm * (r.px * r.px + r.py * r.py) / 2.0;
 }
 
+/* The exact kernels' forms of the drift and the radiating kicks, on doubles:
+ * the expressions above with their divisions taken from the reciprocals at
+ * hand (atb_rn.h), the same IEEE results without a seed, a range test or a
+ * slow branch per division.  `ok` is cleared when an operand leaves the range
+ * in which that holds (tiny or huge numerators, |delta| above 1/8, a path
+ * factor further than 2^-8 from one, an energy loss above 2^-20 in one kick,
+ * anything not finite); the caller then tracks the magnet again by the plain
+ * expressions. */
+
+/* fastdrift: od2 = 2(1 + delta), hp = RN(1/(1 + delta))/2 */
+__device__ __forceinline__ void fastdrift_rn(P6T<double>& r, double nl, double od2, double hp,
+                                             bool& ok) {
+    r.x = r.x + nl * r.px;
+    r.y = r.y + nl * r.py;
+    const double s = r.px * r.px + r.py * r.py;
+    ok &= rn_fit(s);
+    r.ct += rn_div(nl * s, od2, hp);
+}
+
+/* the kick of str_kick_rad_pn / bnd_kick_rad_pn; o = 1 + delta and
+ * pn = RN(1/o) enter and leave with the momentum before and after the loss */
+template <bool BEND, class PL>
+__device__ __forceinline__ void kick_rad_rn(P6T<double>& r, const PL& pl, double L, double irho,
+                                            double lirho, double radc, double& o, double& pn,
+                                            bool& ok) {
+    double re, im;
+    pl.field(r.x, r.y, re, im);
+    const double xpr = r.px * pn, ypr = r.py * pn;
+    const double xx = xpr * xpr, yy = ypr * ypr;
+    const double hx = BEND ? 1.0 + r.x * irho : 1.0;
+    const double d = (BEND ? hx * hx + xx : 1.0 + xx) + yy;
+    const double v_norm2 = rn_rcp_near(d);
+    const double bx = im, by = BEND ? re + irho : re;
+    const double cr = bx * ypr - by * xpr;
+    double b2p;
+    if (BEND)
+        b2p = ((by * hx) * (by * hx) + (bx * hx) * (bx * hx) + cr * cr) * v_norm2;
+    else
+        b2p = (by * by + bx * bx + cr * cr) * v_norm2;
+    const double p2 = pn * pn;
+    const double factor = rn_div(hx + (xx + yy) / 2.0, p2, rn_rcp_step(p2, o * o)) * L;
+    const double dp_0 = r.dp;
+    r.dp -= radc * b2p * factor;
+    o = 1.0 + r.dp;
+    double e;
+    pn = rn_rcp_from(o, pn, &e);
+    ok &= rn_near_fits(d) && rn_below(e, ATB_RN_SEED_HI) && rn_opd_fits(o) &&
+          !rn_below_one(o) && rn_fit(xpr) && rn_fit(ypr);
+    r.px = rn_div(xpr, pn, o);
+    r.py = rn_div(ypr, pn, o);
+    if (BEND) {
+        r.px -= L * (re - (dp_0 - r.x * irho) * irho);
+        r.py = r.py + L * im;
+        r.ct = r.ct + lirho * r.x;
+    } else {
+        r.px = r.px - L * re;
+        r.py = r.py + L * im;
+    }
+}
+
 /* The fast kernels' radiating integrator.  Inside a radiating magnet they
  * carry the angles x' = px/(1+delta), y' = py/(1+delta) in place of px, py:
  * the reference's drift (diff_drift.c:30-43) advances x by L x', y by L y'
@@ -495,6 +566,17 @@ __device__ __forceinline__ void lin_fringe_map(P6T<T>& r, const double* m) {
     r.py = m[6] * y + m[7] * py;
 }
 
+/* An edge without fringe correction: the tangent's argument, edge -
+ * 0/(1+delta), is the edge angle itself whenever 1+delta is finite and not
+ * zero.  The exact kernels test that (the dual-number ones keep the quotient
+ * for its derivative). */
+template <bool FAST, class T>
+__device__ __forceinline__ bool plain_edge(const P6T<T>& r, bool fc0) {
+    if constexpr (FAST) return fc0;
+    else if constexpr (is_dual<T>::value) return false;
+    else return fc0 && isfinite(r.dp) && r.dp != -1.0;
+}
+
 /* Edge focusing of BndMPoleSymplectic4Pass: atphyslib.c:15-79
  * (edge_fringe_entrance / edge_fringe_exit).  sgn = +1 entrance, -1 exit.
  * fy_c = irho*tan(edge) is used whenever the tangent's argument is exactly
@@ -509,7 +591,7 @@ __device__ __forceinline__ void edge_fringe(P6T<T>& r, double irho, double edge,
         T q = r.px / (1 + r.dp);
         fy = irho * tan(sgn > 0 ? (edge - fc + q) : (edge - fc - q));
     } else {
-        if (FAST && fc0) {
+        if (plain_edge<FAST>(r, fc0)) {
             if (method == ATB_BM_2) fy = fy_c / (1 + r.dp); else fy = T(fy_c);
         } else {
             T t = edge - fc / (1 + r.dp);
@@ -535,7 +617,7 @@ __device__ __forceinline__ void edge_fringe_rad(P6T<T>& r, double irho, double e
     if (method == ATB_BM_3) {
         fy = irho * tan(edge - psi + sgn * r.px * p_norm);
     } else {
-        if (FAST && fc0) {
+        if (plain_edge<FAST>(r, fc0)) {
             if (method == ATB_BM_2) fy = fy_c * p_norm; else fy = T(fy_c);
         } else {
             T t = edge - psi * p_norm;

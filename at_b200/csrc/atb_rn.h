@@ -1,0 +1,133 @@
+/*
+ * Correctly rounded quotients and reciprocals from a reciprocal at hand.
+ *
+ * The exact kernels must round every division of the reference's expressions
+ * as IEEE does.  Inside a magnet the divisors are 1 + delta, its rounded
+ * reciprocal, their squares and numbers near one, whose reciprocals are known
+ * already or one short series away, so a quotient needs no seed instruction,
+ * no range test and no slow branch of its own: a product, the remainder (exact
+ * in one fused operation) and one correction,
+ *
+ *     q0 = RN(a y),  r = b q0 - a,  q = RN(q0 - r y),
+ *
+ * the step proved by P. Markstein (IBM J. Res. Dev. 34, 1990: with y = RN(1/b)
+ * and q0 next to a/b, q = RN(a/b)), used for a divisor known in advance as by
+ * Brisebarre, Muller and Raina (IEEE Trans. Comput. 53, 2004).
+ *
+ * Why each use here is exact (u = 2^-53, o = RN(1 + delta), p = RN(1/o)).
+ * A quotient a/b of two doubles is at least ulp(b) / (2 b) ulp(q) away from
+ * any midpoint of the q grid; near a midpoint |r| is half an ulp of q times b.
+ * The corrected value errs by |r| |y - 1/b| before its last rounding, so it
+ * rounds as a/b does when  b^2 |y - 1/b| < ulp(b):
+ *   - y = RN(1/b) (rn_div with y = p, b = o, or both scaled by two):
+ *     |y - 1/b| <= ulp(y) / 2, and b^2 ulp(y) / 2 is below ulp(b) for every b
+ *     in (1/2, 1) and (1, 2).
+ *   - b = p, y = o (rn_div(a, p, o)): |o - 1/p| <= o^2 ulp(p) / 2, and
+ *     b^2 o^2 ulp(p) / 2 = ulp(p) / 2.
+ *   - b = RN(p p), y one step from RN(o o) (rn_rcp_step): within
+ *     (1/2 + 2^-49) ulp of 1/b, which suffices for b > 1 and for b below
+ *     1 - 2^-49; between, b = 1 - 4 i u (p = 1 - 2 i u there) has a reciprocal
+ *     far from any midpoint, so y = RN(1/b).
+ * The remainder is exact, or the quotient lies more than an ulp and less than
+ * one and a half from q0, where rounding it in its last bit changes nothing.
+ * A reciprocal's last step, y + y (1 - d y), is exact for y next to 1/d unless
+ * d's significand is all ones (Markstein); for d near one that is the single
+ * number 1 - u, which the callers exclude.
+ * No step may underflow or overflow: the callers bound the operands and send
+ * everything else through the plain divisions.
+ *
+ * The functions compile for the host as well, where the CPU tests compare
+ * them with the hardware's division.
+ */
+#ifndef ATB_RN_H
+#define ATB_RN_H
+
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#ifdef __CUDACC__
+#define ATB_RN_FN __host__ __device__ __forceinline__
+#else
+#define ATB_RN_FN static inline
+#endif
+
+/* high and low words of a double's bits */
+ATB_RN_FN uint32_t rn_hi(double v) {
+#ifdef __CUDA_ARCH__
+    return (uint32_t)__double2hiint(v);
+#else
+    uint64_t b;
+    memcpy(&b, &v, 8);
+    return (uint32_t)(b >> 32);
+#endif
+}
+ATB_RN_FN uint32_t rn_lo(double v) {
+#ifdef __CUDA_ARCH__
+    return (uint32_t)__double2loint(v);
+#else
+    uint64_t b;
+    memcpy(&b, &v, 8);
+    return (uint32_t)b;
+#endif
+}
+
+/* ---- conditions --------------------------------------------------------- */
+
+/* v in [lo, hi) for positive bounds whose low words are zero */
+ATB_RN_FN bool rn_within(double v, uint32_t lo_hi, uint32_t hi_hi) {
+    return rn_hi(v) - lo_hi < hi_hi - lo_hi;
+}
+/* |v| below the positive bound of high word hi_hi (NaN: no) */
+ATB_RN_FN bool rn_below(double v, uint32_t hi_hi) {
+    return (rn_hi(v) & 0x7fffffffu) < hi_hi;
+}
+/* the quotient's numerator neither underflows nor overflows its remainder:
+   zero, or 2^-900 <= |v| < 2^900 */
+ATB_RN_FN bool rn_fit(double v) {
+    const uint32_t h = rn_hi(v) & 0x7fffffffu;
+    const bool zero = (h | rn_lo(v)) == 0u;
+    return h - 0x07b00000u < 0x78300000u - 0x07b00000u || zero;
+}
+/* 1 - 2^-53, the all-ones significand next to one */
+ATB_RN_FN bool rn_below_one(double v) {
+    return rn_hi(v) == 0x3fefffffu && rn_lo(v) == 0xffffffffu;
+}
+/* 1 + delta in [7/8, 9/8) */
+ATB_RN_FN bool rn_opd_fits(double o) { return rn_within(o, 0x3fec0000u, 0x3ff20000u); }
+/* a divisor of rn_rcp_near in [1 - 2^-8, 1 + 2^-8) */
+ATB_RN_FN bool rn_near_fits(double d) {
+    return rn_within(d, 0x3fefe000u, 0x3ff01000u) && !rn_below_one(d);
+}
+
+/* ---- arithmetic --------------------------------------------------------- */
+
+/* RN(a / b) from y (see above); zeros keep the quotient's sign */
+ATB_RN_FN double rn_div(double a, double b, double y) {
+    const double q = a * y;
+    const double r = fma(b, q, -a);
+    return fma(-r, y, q);
+}
+
+/* one Newton step of the reciprocal of d */
+ATB_RN_FN double rn_rcp_step(double d, double y) { return fma(fma(-d, y, 1.0), y, y); }
+
+/* RN(1 / o) from the reciprocal `seed` of a neighbouring number; e = 1 - o seed
+   must be below 2^-20 (the series drops e^3) and o not 1 - 2^-53 */
+ATB_RN_FN double rn_rcp_from(double o, double seed, double* e) {
+    const double d = fma(-o, seed, 1.0);
+    *e = d;
+    return rn_rcp_step(o, fma(seed, fma(d, d, d), seed));
+}
+#define ATB_RN_SEED_HI 0x3eb00000u   /* 2^-20 */
+
+/* RN(1 / d) for d within 2^-8 of one, from 2 - d: its residue (d - 1)^2 in a
+   geometric series to the third power */
+ATB_RN_FN double rn_rcp_near(double d) {
+    const double y = 2.0 - d;
+    const double r = fma(-d, y, 1.0);
+    const double t = fma(fma(r, r, r), r, r);
+    return rn_rcp_step(d, fma(y, t, y));
+}
+
+#endif /* ATB_RN_H */

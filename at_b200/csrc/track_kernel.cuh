@@ -275,6 +275,155 @@ __device__ __forceinline__ void multipole_steps_generic(P6T<T>* r, const Rec& e,
     }
 }
 
+/* The Forest-Ruth steps of a thick multipole by the reference's plain
+ * expressions (StrMPoleSymplectic4Pass.c:73-93 and the Bnd and Rad variants);
+ * pn0: 1/(1+delta) of the element's entry, which scales the drift lengths of
+ * the non-radiating variants. */
+template <int NP, bool BEND, bool RAD, class PL, class T>
+__device__ __forceinline__ void multipole_steps_plain(P6T<T>* r, const Rec& e, const PL& pl,
+                                                      const T* nl1, const T* nl2, double irho,
+                                                      int ns) {
+    const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
+    const double k1i = BEND ? e.f(ATB_BM_K1IRHO) : 0.0, k2i = BEND ? e.f(ATB_BM_K2IRHO) : 0.0;
+    if (RAD) {
+        const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2), radc = e.f(ATB_SM_RADC);
+        /* pn: 1/(1+delta) as the reference last evaluated it (it changes
+           only in a kick's energy loss, and the kick hands it on) */
+        T pn[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) pn[k] = 1.0 / (1.0 + r[k].dp);
+        for (int m = 0; m < ns; ++m) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                diff_drift_pn(r[k], L1, pn[k]);
+                if (BEND) bnd_kick_rad_pn(r[k], pl, K1, irho, k1i, radc, pn[k]);
+                else str_kick_rad_pn(r[k], pl, K1, radc, pn[k]);
+                diff_drift_pn(r[k], L2, pn[k]);
+                if (BEND) bnd_kick_rad_pn(r[k], pl, K2, irho, k2i, radc, pn[k]);
+                else str_kick_rad_pn(r[k], pl, K2, radc, pn[k]);
+                diff_drift_pn(r[k], L2, pn[k]);
+                if (BEND) bnd_kick_rad_pn(r[k], pl, K1, irho, k1i, radc, pn[k]);
+                else str_kick_rad_pn(r[k], pl, K1, radc, pn[k]);
+                diff_drift_pn(r[k], L1, pn[k]);
+            }
+        }
+    } else {
+        for (int m = 0; m < ns; ++m) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                fastdrift<false>(r[k], nl1[k], T(0.0));
+                if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
+                fastdrift<false>(r[k], nl2[k], T(0.0));
+                if (BEND) bndthinkick(r[k], pl, K2, irho, k2i); else strthinkick(r[k], pl, K2);
+                fastdrift<false>(r[k], nl2[k], T(0.0));
+                if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
+                fastdrift<false>(r[k], nl1[k], T(0.0));
+            }
+        }
+    }
+}
+
+/* The same out of line, for the rare magnet whose operands leave the range of
+ * multipole_steps_rn. */
+template <bool BEND, bool RAD>
+__device__ __noinline__ P6 multipole_steps_call(P6 r, Rec e, Param pm, double nl1, double nl2) {
+    const int mo = e.mo();
+    const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
+    Poly<-1> pl;
+    pl.load(A, A + mo + 1, mo);
+    if (pm.k >= 0) pl.set_param(pm.k, pm.v);
+    multipole_steps_plain<1, BEND, RAD>(&r, e, pl, &nl1, &nl2, BEND ? e.f(ATB_BM_IRHO) : 0.0,
+                                        e.nsteps());
+    return r;
+}
+
+/* multipole_steps_plain on doubles in the exact kernels, with the divisions
+ * of atb_rn.h: the same IEEE results, straight-line code in the step loop.
+ * The divisions bounded these loops: about nine FP64 instructions each, a
+ * seed on the XU pipe and a branch to a slow path that ended the block the
+ * compiler could interleave (a plain sextupole step of a lone warp took 631
+ * cycles and takes 289, a radiating one 1886 and 1165; with 16 warps a
+ * scheduler 296 and 197, 836 and 563 cycles a warp).  A warp with an operand
+ * out of range pays for both loops, which only particles about to be lost
+ * do. */
+template <int NP, bool BEND, bool RAD, class PL>
+__device__ __forceinline__ void multipole_steps_rn(P6* r, const Rec& e, const PL& pl,
+                                                   const Param& pm, const double* pn0,
+                                                   const double* dp0, const double* nl1, const double* nl2,
+                                                   double irho, int ns) {
+    const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
+    const double k1i = BEND ? e.f(ATB_BM_K1IRHO) : 0.0, k2i = BEND ? e.f(ATB_BM_K2IRHO) : 0.0;
+    P6 in[NP];
+    bool ok[NP];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) in[k] = r[k];
+    if (RAD) {
+        const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2), radc = e.f(ATB_SM_RADC);
+        double o[NP], pn[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            o[k] = 1.0 + r[k].dp;
+            pn[k] = 1.0 / o[k];
+            ok[k] = rn_opd_fits(o[k]);
+        }
+        for (int m = 0; m < ns; ++m) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) diff_drift_pn(r[k], L1, pn[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k)
+                kick_rad_rn<BEND>(r[k], pl, K1, irho, k1i, radc, o[k], pn[k], ok[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) diff_drift_pn(r[k], L2, pn[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k)
+                kick_rad_rn<BEND>(r[k], pl, K2, irho, k2i, radc, o[k], pn[k], ok[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) diff_drift_pn(r[k], L2, pn[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k)
+                kick_rad_rn<BEND>(r[k], pl, K1, irho, k1i, radc, o[k], pn[k], ok[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) diff_drift_pn(r[k], L1, pn[k]);
+        }
+    } else {
+        double od2[NP], hp[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            const double o = 1.0 + r[k].dp;
+            od2[k] = 2.0 * o;
+            hp[k] = 0.5 * pn0[k];
+            /* delta may have changed since pn0 (an entrance shift of it) */
+            ok[k] = rn_opd_fits(o) && r[k].dp == dp0[k] && rn_fit(nl1[k]) && rn_fit(nl2[k]) &&
+                    rn_below(r[k].x, 0x7ff00000u) && rn_below(r[k].y, 0x7ff00000u);
+        }
+        for (int m = 0; m < ns; ++m) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) fastdrift_rn(r[k], nl1[k], od2[k], hp[k], ok[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) fastdrift_rn(r[k], nl2[k], od2[k], hp[k], ok[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bndthinkick(r[k], pl, K2, irho, k2i); else strthinkick(r[k], pl, K2);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) fastdrift_rn(r[k], nl2[k], od2[k], hp[k], ok[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) fastdrift_rn(r[k], nl1[k], od2[k], hp[k], ok[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NP; ++k)
+        if (!ok[k]) r[k] = multipole_steps_call<BEND, RAD>(in[k], e, pm, nl1[k], nl2[k]);
+}
+
 /* StrMPoleSymplectic4Pass.c:29-109, BndMPoleSymplectic4Pass.c:38-129,
  * StrMPoleSymplectic4RadPass.c:30-115, BndMPoleSymplectic4RadPass.c:39-128.
  * NP particles of one thread pass the element together: every per-particle
@@ -294,14 +443,17 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, const Rec& e, const 
     pl.load(A, B, mo);
     if (pm.k >= 0) pl.set_param(pm.k, pm.v);
 
-    T nl1[NP], nl2[NP];
+    T pn0[NP], dp0[NP], nl1[NP], nl2[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         if (fl & ATB_F_SCALING) change_pref<kFast>(r[k], e.f(ATB_SM_SCALE));
+        pn0[k] = 0.0;
+        dp0[k] = r[k].dp;
         nl1[k] = 0.0;
         nl2[k] = 0.0;
         if (!RAD) {
             T p_norm = 1.0 / (1.0 + r[k].dp);
+            pn0[k] = p_norm;
             nl1[k] = L1 * p_norm;
             nl2[k] = L2 * p_norm;
         }
@@ -345,6 +497,10 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, const Rec& e, const 
         /* another integrator of the GPU call: steps of SL*c[i] drift and
            SL*d[i] kick (atgpu/SymplecticIntegrator.cpp:140-171) */
         multipole_steps_generic<NP, BEND, RAD>(r, e, pl, nl2, irho, ns);
+    } else if constexpr (is_dual<T>::value) {
+        multipole_steps_plain<NP, BEND, RAD>(r, e, pl, nl1, nl2, irho, ns);
+    } else if constexpr (!kFast) {
+        multipole_steps_rn<NP, BEND, RAD>(r, e, pl, pm, pn0, dp0, nl1, nl2, irho, ns);
     } else if (RAD) {
         const double radc = e.f(ATB_SM_RADC);
         if constexpr (kFast && !is_dual<T>::value) {
@@ -386,27 +542,6 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, const Rec& e, const 
                 for (int k = 0; k < NP; ++k) {
                     r[k].px = a[k].xp * a[k].opd;
                     r[k].py = a[k].yp * a[k].opd;
-                }
-            }
-        } else {
-            /* pn: 1/(1+delta) as the reference last evaluated it (it changes
-               only in a kick's energy loss, and the kick hands it on) */
-            T pn[NP];
-#pragma unroll
-            for (int k = 0; k < NP; ++k) pn[k] = 1.0 / (1.0 + r[k].dp);
-            for (int m = 0; m < ns; ++m) {
-#pragma unroll
-                for (int k = 0; k < NP; ++k) {
-                    diff_drift_pn(r[k], L1, pn[k]);
-                    if (BEND) bnd_kick_rad_pn(r[k], pl, K1, irho, k1i, radc, pn[k]);
-                    else str_kick_rad_pn(r[k], pl, K1, radc, pn[k]);
-                    diff_drift_pn(r[k], L2, pn[k]);
-                    if (BEND) bnd_kick_rad_pn(r[k], pl, K2, irho, k2i, radc, pn[k]);
-                    else str_kick_rad_pn(r[k], pl, K2, radc, pn[k]);
-                    diff_drift_pn(r[k], L2, pn[k]);
-                    if (BEND) bnd_kick_rad_pn(r[k], pl, K1, irho, k1i, radc, pn[k]);
-                    else str_kick_rad_pn(r[k], pl, K1, radc, pn[k]);
-                    diff_drift_pn(r[k], L1, pn[k]);
                 }
             }
         }
@@ -495,21 +630,20 @@ __device__ __forceinline__ void pass_multipole_dispatch_n(P6T<T>* r, const Rec& 
                 return;
             }
         }
-        /* the fast kernels evaluate upright magnets' fields without the
-           zero skew terms */
-        const bool upright = kFast && (e.flags() & ATB_F_NOSKEW);
+        /* upright magnets' fields without the zero skew terms */
+        const bool upright = e.flags() & ATB_F_NOSKEW;
         switch (e.mo()) {
             case 0: pass_multipole_n<NP, 0, BEND, RAD>(r, e, pm); break;
             case 1:
-                if (upright) pass_multipole_n<NP, 1, BEND, RAD, !kFast>(r, e, pm);
+                if (upright) pass_multipole_n<NP, 1, BEND, RAD, false>(r, e, pm);
                 else pass_multipole_n<NP, 1, BEND, RAD>(r, e, pm);
                 break;
             case 2:
-                if (upright) pass_multipole_n<NP, 2, BEND, RAD, !kFast>(r, e, pm);
+                if (upright) pass_multipole_n<NP, 2, BEND, RAD, false>(r, e, pm);
                 else pass_multipole_n<NP, 2, BEND, RAD>(r, e, pm);
                 break;
             case 3:
-                if (upright) pass_multipole_n<NP, 3, BEND, RAD, !kFast>(r, e, pm);
+                if (upright) pass_multipole_n<NP, 3, BEND, RAD, false>(r, e, pm);
                 else pass_multipole_n<NP, 3, BEND, RAD>(r, e, pm);
                 break;
             default: pass_multipole_n<NP, -1, BEND, RAD>(r, e, pm); break;
@@ -678,6 +812,15 @@ __device__ __forceinline__ void pass_multipoles_together(P6 (&r)[NP], const Rec&
 /* pyat/at.c:123: lost if any coordinate is non-finite or |r_n| > 1, n < 5 */
 template <class T>
 __device__ __forceinline__ bool is_bad(const P6T<T>& r) {
+    if constexpr (!is_dual<T>::value) {
+        /* nearly always every |r_n| < 1 and ct is finite, which the exponents
+           show without a floating-point compare */
+        const uint32_t m = 0x7fffffffu;
+        const uint32_t a = max(rn_hi(r.x) & m, rn_hi(r.px) & m);
+        const uint32_t b = max(rn_hi(r.y) & m, rn_hi(r.py) & m);
+        if (max(max(a, b), rn_hi(r.dp) & m) < 0x3ff00000u && rn_below(r.ct, 0x7ff00000u))
+            return false;
+    }
     return !all_finite(r) || fabs(val(r.x)) > 1.0 || fabs(val(r.px)) > 1.0 ||
            fabs(val(r.y)) > 1.0 || fabs(val(r.py)) > 1.0 || fabs(val(r.dp)) > 1.0;
 }
