@@ -515,7 +515,8 @@ __device__ __forceinline__ Lam6 adj_dual(const P6& s, const Lam6& in, const Rec&
     r.py = D(s.py); r.dp = D(s.dp); r.ct = D(s.ct);
     r.x.d[0] = 1.0; r.px.d[1] = 1.0; r.y.d[2] = 1.0;
     r.py.d[3] = 1.0; r.dp.d[4] = 1.0; r.ct.d[5] = 1.0;
-    track_element(r, e, nturn, pm);
+    NoRecip<D> none;
+    track_element(r, none, e, nturn, pm);
     const D* rows[6] = {&r.x, &r.px, &r.y, &r.py, &r.dp, &r.ct};
     Lam6 out;
 #pragma unroll
@@ -596,6 +597,7 @@ atb_adjoint_forward_kernel(const AtbAdjoint A) {
     P6 r;
     load6(A.r + 6 * p, r);
     bool lost = isnan(r.x);
+    Recip rc;
     for (int tt = 0; tt < A.nturns; ++tt) {
         if (A.ckpt && tt % A.stride == 0)
             store6(A.ckpt + 6 * ((long long)(tt / A.stride) * A.ld + p), r);
@@ -604,7 +606,7 @@ atb_adjoint_forward_kernel(const AtbAdjoint A) {
         for (int ei = 0; ei < A.nelem; ++ei) {
             if (A.scratch)
                 store6(A.scratch + 6 * (((long long)tt * A.nelem + ei) * A.ld + p), r);
-            track_element(r, adj_rec(A, ei), nturn, adj_param(A, ei));
+            track_element(r, rc, adj_rec(A, ei), nturn, adj_param(A, ei));
             if (is_bad(r)) {                  /* pyat/at.c:115-139 */
                 lost = true;
                 break;
@@ -645,10 +647,11 @@ atb_adjoint_turn_kernel(const AtbAdjoint A) {
         if (live) live = !isnan(__ldg(A.next + 6 * p));
     } else {
         /* the turn once more, every element's entry state to the scratch */
+        Recip rc;
         for (int ei = 0; ei < A.nelem; ++ei) {
             if (live) {
                 store6(A.scratch + 6 * ((long long)ei * np + p), s);
-                track_element(s, adj_rec(A, ei), A.turn0, adj_param(A, ei));
+                track_element(s, rc, adj_rec(A, ei), A.turn0, adj_param(A, ei));
                 if (is_bad(s)) live = false;      /* lost in this turn */
             }
         }

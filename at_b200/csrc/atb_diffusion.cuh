@@ -273,7 +273,8 @@ atb_element_maps_kernel(const AtbElemMaps A) {
         r.py = TD(o[3]); r.dp = TD(o[4]); r.ct = TD(o[5]);
         r.x.d[0] = 1.0; r.px.d[1] = 1.0; r.y.d[2] = 1.0;
         r.py.d[3] = 1.0; r.dp.d[4] = 1.0; r.ct.d[5] = 1.0;
-        track_element(r, e, 0);
+        NoRecip<TD> none;
+        track_element(r, none, e, 0);
         TD* rows[6] = ATB_ROWS(r);
         if (A.m66) {
             double* m = A.m66 + 36 * (long long)i;

@@ -136,22 +136,25 @@ __device__ __forceinline__ void change_pref(P6T<T>& r, double s) {
 }
 
 /* atlalib.c:59-68 ATdrift6 == driftkickrad.c:36-45 drift6 == diff_drift.c:30-43
- * (without the diffusion-matrix branch) */
+ * (without the diffusion-matrix branch); pn = 1/(1+delta) */
 template <bool FAST, class T>
-__device__ __forceinline__ void drift6(P6T<T>& r, double L) {
+__device__ __forceinline__ void drift6_pn(P6T<T>& r, double L, const T& pn) {
+    const T nl = L * pn;
     if constexpr (FAST) {
-        double pn = 1.0 / (1.0 + r.dp);
-        double nl = L * pn;
         r.x += nl * r.px;
         r.y += nl * r.py;
         r.ct += (0.5 * nl * pn) * (r.px * r.px + r.py * r.py);
     } else {
-        T pn = 1 / (1 + r.dp);
-        T nl = L * pn;
         r.x = madd(r.x, nl, r.px);
         r.y = madd(r.y, nl, r.py);
         r.ct += nl * pn * (r.px * r.px + r.py * r.py) / 2;
     }
+}
+
+template <bool FAST, class T>
+__device__ __forceinline__ void drift6(P6T<T>& r, double L) {
+    const T pn = 1.0 / (1.0 + r.dp);
+    drift6_pn<FAST>(r, L, pn);
 }
 
 /* driftkick.c:37-48 fastdrift.  FAST: c2 = NormL/(2(1+delta)) precomputed. */
@@ -406,19 +409,40 @@ __device__ __forceinline__ void diff_drift_pn(P6T<T>& r, double L, const T& pn) 
  * the expressions above with their divisions taken from the reciprocals at
  * hand (atb_rn.h), the same IEEE results without a seed, a range test or a
  * slow branch per division.  `ok` is cleared when an operand leaves the range
- * in which that holds (tiny or huge numerators, |delta| above 1/8, a path
- * factor further than 2^-8 from one, an energy loss above 2^-20 in one kick,
- * anything not finite); the caller then tracks the magnet again by the plain
- * expressions. */
+ * in which that holds (tiny numerators, angles above 31 mrad or a path factor
+ * further than 2^-8 from one, an energy loss above 2^-20 in one kick, anything
+ * not finite), tested on exponents with integer instructions; the caller then
+ * tracks the magnet again by the plain expressions. */
+
+/* what a drift adds to x, y and ct (to ct twice that in a radiating magnet,
+ * whose drift halves the last product: ct + w/2 is one fused operation, w/2
+ * being exact) */
+struct DriftInc {
+    double x, y, ct;
+};
+__device__ __forceinline__ void add_drift(P6T<double>& r, const DriftInc& d) {
+    r.x += d.x;
+    r.y += d.y;
+    r.ct += d.ct;
+}
+__device__ __forceinline__ void add_drift_rad(P6T<double>& r, const DriftInc& d) {
+    r.x += d.x;
+    r.y += d.y;
+    r.ct = fma(0.5, d.ct, r.ct);
+}
 
 /* fastdrift: od2 = 2(1 + delta), hp = RN(1/(1 + delta))/2 */
-__device__ __forceinline__ void fastdrift_rn(P6T<double>& r, double nl, double od2, double hp,
-                                             bool& ok) {
-    r.x = r.x + nl * r.px;
-    r.y = r.y + nl * r.py;
+__device__ __forceinline__ DriftInc fastdrift_inc(const P6T<double>& r, double nl, double od2,
+                                                  double hp, bool& ok) {
     const double s = r.px * r.px + r.py * r.py;
-    ok &= rn_fit(s);
-    r.ct += rn_div(nl * s, od2, hp);
+    ok &= rn_square_fits(s);
+    return DriftInc{nl * r.px, nl * r.py, rn_div(nl * s, od2, hp)};
+}
+
+/* diff_drift_pn */
+__device__ __forceinline__ DriftInc drift_rad_inc(const P6T<double>& r, double L, double pn) {
+    const double nl = L * pn;
+    return DriftInc{nl * r.px, nl * r.py, nl * pn * (r.px * r.px + r.py * r.py)};
 }
 
 /* the kick of str_kick_rad_pn / bnd_kick_rad_pn; o = 1 + delta and
@@ -433,7 +457,7 @@ __device__ __forceinline__ void kick_rad_rn(P6T<double>& r, const PL& pl, double
     const double xx = xpr * xpr, yy = ypr * ypr;
     const double hx = BEND ? 1.0 + r.x * irho : 1.0;
     const double d = (BEND ? hx * hx + xx : 1.0 + xx) + yy;
-    const double v_norm2 = rn_rcp_near(d);
+    const double v_norm2 = BEND ? rn_rcp_near(d) : rn_rcp_nearer(d);
     const double bx = im, by = BEND ? re + irho : re;
     const double cr = bx * ypr - by * xpr;
     double b2p;
@@ -442,14 +466,14 @@ __device__ __forceinline__ void kick_rad_rn(P6T<double>& r, const PL& pl, double
     else
         b2p = (by * by + bx * bx + cr * cr) * v_norm2;
     const double p2 = pn * pn;
-    const double factor = rn_div(hx + (xx + yy) / 2.0, p2, rn_rcp_step(p2, o * o)) * L;
+    const double factor = rn_div(fma(0.5, xx + yy, hx), p2, rn_rcp_step(p2, o * o)) * L;
     const double dp_0 = r.dp;
     r.dp -= radc * b2p * factor;
     o = 1.0 + r.dp;
     double e;
     pn = rn_rcp_from(o, pn, &e);
-    ok &= rn_near_fits(d) && rn_below(e, ATB_RN_SEED_HI) && rn_opd_fits(o) &&
-          !rn_below_one(o) && rn_fit(xpr) && rn_fit(ypr);
+    ok &= (BEND ? rn_near_fits(d) : rn_nearer_fits(d)) && rn_below(e, ATB_RN_SEED_HI) &&
+          !rn_below_one(o) && rn_not_tiny(xpr) && rn_not_tiny(ypr);
     r.px = rn_div(xpr, pn, o);
     r.py = rn_div(ypr, pn, o);
     if (BEND) {

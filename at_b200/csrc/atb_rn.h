@@ -82,22 +82,38 @@ ATB_RN_FN bool rn_within(double v, uint32_t lo_hi, uint32_t hi_hi) {
 ATB_RN_FN bool rn_below(double v, uint32_t hi_hi) {
     return (rn_hi(v) & 0x7fffffffu) < hi_hi;
 }
-/* the quotient's numerator neither underflows nor overflows its remainder:
-   zero, or 2^-900 <= |v| < 2^900 */
-ATB_RN_FN bool rn_fit(double v) {
+/* a coordinate: zero, or 2^-400 <= |v| < 2^900 */
+ATB_RN_FN bool rn_coord_fits(double v) {
     const uint32_t h = rn_hi(v) & 0x7fffffffu;
-    const bool zero = (h | rn_lo(v)) == 0u;
-    return h - 0x07b00000u < 0x78300000u - 0x07b00000u || zero;
+    return h - 0x26f00000u < 0x78300000u - 0x26f00000u || (h | rn_lo(v)) == 0u;
 }
 /* 1 - 2^-53, the all-ones significand next to one */
 ATB_RN_FN bool rn_below_one(double v) {
     return rn_hi(v) == 0x3fefffffu && rn_lo(v) == 0xffffffffu;
 }
-/* 1 + delta in [7/8, 9/8) */
-ATB_RN_FN bool rn_opd_fits(double o) { return rn_within(o, 0x3fec0000u, 0x3ff20000u); }
+/* 1 + delta within 7/64 of one: 4096 steps of three kicks that each change it
+   by 2^-20 at most leave it in [7/8, 9/8) */
+ATB_RN_FN bool rn_opd_fits(double o) { return rn_within(o, 0x3fec8000u, 0x3ff1c000u); }
 /* a divisor of rn_rcp_near in [1 - 2^-8, 1 + 2^-8) */
 ATB_RN_FN bool rn_near_fits(double d) {
     return rn_within(d, 0x3fefe000u, 0x3ff01000u) && !rn_below_one(d);
+}
+/* a divisor of rn_rcp_nearer in [1, 1 + 2^-10) */
+ATB_RN_FN bool rn_nearer_fits(double d) { return rn_within(d, 0x3ff00000u, 0x3ff00400u); }
+/* a length: zero, or 2^-40 <= |v| < 2^40 */
+ATB_RN_FN bool rn_length_fits(double v) {
+    const uint32_t h = rn_hi(v) & 0x7fffffffu;
+    return h - 0x3d700000u < 0x42700000u - 0x3d700000u || (h | rn_lo(v)) == 0u;
+}
+/* The two tests of the step loops, where only tiny nonzero values are left to
+   exclude.  A denormal with a zero high word passes as zero; none comes up from
+   coordinates that passed rn_coord_fits. */
+/* v >= 0: zero or at least 2^-860 */
+ATB_RN_FN bool rn_square_fits(double v) { return rn_hi(v) - 1u >= 0x0a300000u - 1u; }
+/* |v| zero or at least 2^-480 */
+ATB_RN_FN bool rn_not_tiny(double v) {
+    const uint32_t h = rn_hi(v);
+    return h + h - 2u >= 2u * 0x21f00000u - 2u;
 }
 
 /* ---- arithmetic --------------------------------------------------------- */
@@ -122,7 +138,12 @@ ATB_RN_FN double rn_rcp_from(double o, double seed, double* e) {
 #define ATB_RN_SEED_HI 0x3eb00000u   /* 2^-20 */
 
 /* RN(1 / d) for d within 2^-8 of one, from 2 - d: its residue (d - 1)^2 in a
-   geometric series to the third power */
+   geometric series to the third power, to the second for d within 2^-10 */
+ATB_RN_FN double rn_rcp_nearer(double d) {
+    const double y = 2.0 - d;
+    const double r = fma(-d, y, 1.0);
+    return rn_rcp_step(d, fma(y, fma(r, r, r), y));
+}
 ATB_RN_FN double rn_rcp_near(double d) {
     const double y = 2.0 - d;
     const double r = fma(-d, y, 1.0);

@@ -117,7 +117,8 @@ atb_tangent_kernel(const AtbTangent A) {
             const int q = A.pelem ? A.pelem[ei] : -1;
             Param pm{-1, 0.0};
             if (q >= 0) { pm.k = A.porder[q]; pm.v = A.pvalue[q]; }
-            track_element(r, e, nturn, pm);
+            NoRecip<TD> none;
+            track_element(r, none, e, nturn, pm);
             if (is_bad(r)) {          /* pyat/at.c:115-139 */
                 lost = true;
                 break;

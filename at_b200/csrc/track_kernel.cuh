@@ -19,6 +19,7 @@
 #define ATB_TRACK_KERNEL_CUH
 
 #include <cstdint>
+#include <type_traits>
 #include "atb_physics.cuh"
 #include "atb_integrators.h"
 #include "atb_kernel_api.h"
@@ -177,6 +178,31 @@ __device__ __forceinline__ T fringe_b1(const Rec& e, const Param& pm) {
         if (pm.k == 1) b1 = pm.v;
     }
     return b1;
+}
+
+/* 1/(1+delta) of the momentum it was last asked for.  delta changes only in
+ * cavities and radiating kicks (whose loops leave the new reciprocal here),
+ * so drifts and magnets mostly find theirs without a division.  The dual
+ * numbers of the derivative kernels divide every time. */
+struct Recip {
+    double dp, pn;
+    __device__ __forceinline__ Recip() : dp(nan_d()), pn(0.0) {}
+};
+template <class T>
+struct NoRecip {};
+template <class T>
+using RecipOf = typename std::conditional<is_dual<T>::value, NoRecip<T>, Recip>::type;
+
+__device__ __forceinline__ double opd_rcp(Recip& c, double dp) {
+    if (dp != c.dp) {
+        c.dp = dp;
+        c.pn = 1.0 / (1.0 + dp);
+    }
+    return c.pn;
+}
+template <class T>
+__device__ __forceinline__ T opd_rcp(NoRecip<T>&, const T& dp) {
+    return 1.0 / (1.0 + dp);
 }
 
 /* The integration steps of a thick multipole under integrator id
@@ -342,48 +368,70 @@ __device__ __noinline__ P6 multipole_steps_call(P6 r, Rec e, Param pm, double nl
  * The divisions bounded these loops: about nine FP64 instructions each, a
  * seed on the XU pipe and a branch to a slow path that ended the block the
  * compiler could interleave (a plain sextupole step of a lone warp took 631
- * cycles and takes 289, a radiating one 1886 and 1165; with 16 warps a
- * scheduler 296 and 197, 836 and 563 cycles a warp).  A warp with an operand
- * out of range pays for both loops, which only particles about to be lost
- * do. */
+ * cycles and takes 275, a radiating one 1886 and 958; of 16 warps a scheduler
+ * each takes 296 and now 174 cycles a plain step, 836 and 495 a radiating
+ * one).  The last drift of a step and the
+ * first of the next have the same length, momenta and 1/(1+delta), hence the
+ * same increments: they are computed once and added twice.  A warp with an
+ * operand out of range pays for both loops, which only particles about to be
+ * lost do.  Returns 1/(1+delta) at the exit of a radiating magnet. */
 template <int NP, bool BEND, bool RAD, class PL>
-__device__ __forceinline__ void multipole_steps_rn(P6* r, const Rec& e, const PL& pl,
-                                                   const Param& pm, const double* pn0,
-                                                   const double* dp0, const double* nl1, const double* nl2,
+__device__ __forceinline__ void multipole_steps_rn(P6* r, Recip* c, const Rec& e, const PL& pl,
+                                                   const Param& pm, const double* dp0,
+                                                   const double* nl1, const double* nl2,
                                                    double irho, int ns) {
+    if (ns <= 0) return;
     const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
     const double k1i = BEND ? e.f(ATB_BM_K1IRHO) : 0.0, k2i = BEND ? e.f(ATB_BM_K2IRHO) : 0.0;
     P6 in[NP];
     bool ok[NP];
+    DriftInc d1[NP];
 #pragma unroll
-    for (int k = 0; k < NP; ++k) in[k] = r[k];
+    for (int k = 0; k < NP; ++k) {
+        in[k] = r[k];
+        ok[k] = rn_coord_fits(r[k].x) && rn_coord_fits(r[k].px) && rn_coord_fits(r[k].y) &&
+                rn_coord_fits(r[k].py);
+    }
     if (RAD) {
         const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2), radc = e.f(ATB_SM_RADC);
+        const bool uniform = rn_length_fits(L1) && rn_length_fits(L2) && ns <= 4096;
         double o[NP], pn[NP];
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
             o[k] = 1.0 + r[k].dp;
-            pn[k] = 1.0 / o[k];
-            ok[k] = rn_opd_fits(o[k]);
+            pn[k] = opd_rcp(c[k], r[k].dp);
+            ok[k] &= uniform && rn_opd_fits(o[k]);
+            d1[k] = drift_rad_inc(r[k], L1, pn[k]);
+            add_drift_rad(r[k], d1[k]);
         }
-        for (int m = 0; m < ns; ++m) {
-#pragma unroll
-            for (int k = 0; k < NP; ++k) diff_drift_pn(r[k], L1, pn[k]);
+        for (int m = 1;; ++m) {
 #pragma unroll
             for (int k = 0; k < NP; ++k)
                 kick_rad_rn<BEND>(r[k], pl, K1, irho, k1i, radc, o[k], pn[k], ok[k]);
 #pragma unroll
-            for (int k = 0; k < NP; ++k) diff_drift_pn(r[k], L2, pn[k]);
+            for (int k = 0; k < NP; ++k) add_drift_rad(r[k], drift_rad_inc(r[k], L2, pn[k]));
 #pragma unroll
             for (int k = 0; k < NP; ++k)
                 kick_rad_rn<BEND>(r[k], pl, K2, irho, k2i, radc, o[k], pn[k], ok[k]);
 #pragma unroll
-            for (int k = 0; k < NP; ++k) diff_drift_pn(r[k], L2, pn[k]);
+            for (int k = 0; k < NP; ++k) add_drift_rad(r[k], drift_rad_inc(r[k], L2, pn[k]));
 #pragma unroll
             for (int k = 0; k < NP; ++k)
                 kick_rad_rn<BEND>(r[k], pl, K1, irho, k1i, radc, o[k], pn[k], ok[k]);
 #pragma unroll
-            for (int k = 0; k < NP; ++k) diff_drift_pn(r[k], L1, pn[k]);
+            for (int k = 0; k < NP; ++k) {
+                d1[k] = drift_rad_inc(r[k], L1, pn[k]);
+                add_drift_rad(r[k], d1[k]);
+            }
+            if (m == ns) break;
+#pragma unroll
+            for (int k = 0; k < NP; ++k) add_drift_rad(r[k], d1[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            ok[k] &= rn_not_tiny(r[k].px) && rn_not_tiny(r[k].py);
+            c[k].dp = r[k].dp;
+            c[k].pn = pn[k];
         }
     } else {
         double od2[NP], hp[NP];
@@ -391,80 +439,238 @@ __device__ __forceinline__ void multipole_steps_rn(P6* r, const Rec& e, const PL
         for (int k = 0; k < NP; ++k) {
             const double o = 1.0 + r[k].dp;
             od2[k] = 2.0 * o;
-            hp[k] = 0.5 * pn0[k];
-            /* delta may have changed since pn0 (an entrance shift of it) */
-            ok[k] = rn_opd_fits(o) && r[k].dp == dp0[k] && rn_fit(nl1[k]) && rn_fit(nl2[k]) &&
-                    rn_below(r[k].x, 0x7ff00000u) && rn_below(r[k].y, 0x7ff00000u);
+            hp[k] = 0.5 * c[k].pn;
+            /* the cached reciprocal is the entry's: an entrance shift may
+               have changed delta since */
+            ok[k] &= rn_opd_fits(o) && r[k].dp == dp0[k] && rn_length_fits(nl1[k]) &&
+                     rn_length_fits(nl2[k]);
+            d1[k] = fastdrift_inc(r[k], nl1[k], od2[k], hp[k], ok[k]);
+            add_drift(r[k], d1[k]);
         }
-        for (int m = 0; m < ns; ++m) {
-#pragma unroll
-            for (int k = 0; k < NP; ++k) fastdrift_rn(r[k], nl1[k], od2[k], hp[k], ok[k]);
+        for (int m = 1;; ++m) {
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
             }
 #pragma unroll
-            for (int k = 0; k < NP; ++k) fastdrift_rn(r[k], nl2[k], od2[k], hp[k], ok[k]);
+            for (int k = 0; k < NP; ++k)
+                add_drift(r[k], fastdrift_inc(r[k], nl2[k], od2[k], hp[k], ok[k]));
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 if (BEND) bndthinkick(r[k], pl, K2, irho, k2i); else strthinkick(r[k], pl, K2);
             }
 #pragma unroll
-            for (int k = 0; k < NP; ++k) fastdrift_rn(r[k], nl2[k], od2[k], hp[k], ok[k]);
+            for (int k = 0; k < NP; ++k)
+                add_drift(r[k], fastdrift_inc(r[k], nl2[k], od2[k], hp[k], ok[k]));
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
             }
 #pragma unroll
-            for (int k = 0; k < NP; ++k) fastdrift_rn(r[k], nl1[k], od2[k], hp[k], ok[k]);
+            for (int k = 0; k < NP; ++k) {
+                d1[k] = fastdrift_inc(r[k], nl1[k], od2[k], hp[k], ok[k]);
+                add_drift(r[k], d1[k]);
+            }
+            if (m == ns) break;
+#pragma unroll
+            for (int k = 0; k < NP; ++k) add_drift(r[k], d1[k]);
         }
+        /* an overflow anywhere has reached ct */
+#pragma unroll
+        for (int k = 0; k < NP; ++k) ok[k] &= rn_below(r[k].ct, 0x7ff00000u);
     }
 #pragma unroll
     for (int k = 0; k < NP; ++k)
-        if (!ok[k]) r[k] = multipole_steps_call<BEND, RAD>(in[k], e, pm, nl1[k], nl2[k]);
+        if (!ok[k]) {
+            r[k] = multipole_steps_call<BEND, RAD>(in[k], e, pm, nl1[k], nl2[k]);
+            c[k] = Recip();
+        }
+}
+
+/* The fast kernels' steps. */
+template <int NP, bool BEND, bool RAD, class PL>
+__device__ __forceinline__ void multipole_steps_fast(P6* r, Recip* c, const Rec& e, const PL& pl,
+                                                     const double* nl1, const double* nl2,
+                                                     double irho, int ns) {
+    const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
+    const double k1i = BEND ? e.f(ATB_BM_K1IRHO) : 0.0, k2i = BEND ? e.f(ATB_BM_K2IRHO) : 0.0;
+    if (RAD) {
+        if (ns <= 0) return;
+        const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2), radc = e.f(ATB_SM_RADC);
+        const double rk1 = radc * K1, rk2 = radc * K2;
+        const double h1 = 0.5 * L1, h2 = 0.5 * L2;
+        RadAngles a[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            const double pn = opd_rcp(c[k], r[k].dp);
+            a[k] = RadAngles{r[k].px * pn, r[k].py * pn, 0.0, 1.0 + r[k].dp};
+        }
+        for (int m = 0; m < ns; ++m) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L1, h1);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K1, irho, k1i, rk1);
+                else str_kick_rad_fast(r[k], a[k], pl, K1, rk1);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L2, h2);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K2, irho, k2i, rk2);
+                else str_kick_rad_fast(r[k], a[k], pl, K2, rk2);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L2, h2);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K1, irho, k1i, rk1);
+                else str_kick_rad_fast(r[k], a[k], pl, K1, rk1);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L1, h1);
+        }
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            r[k].px = a[k].xp * a[k].opd;
+            r[k].py = a[k].yp * a[k].opd;
+        }
+    } else {
+        double c1[NP], c2[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            const double h = 0.5 * opd_rcp(c[k], r[k].dp);
+            c1[k] = nl1[k] * h;
+            c2[k] = nl2[k] * h;
+        }
+        for (int m = 0; m < ns; ++m) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) fastdrift<kFast>(r[k], nl1[k], c1[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) fastdrift<kFast>(r[k], nl2[k], c2[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bndthinkick(r[k], pl, K2, irho, k2i); else strthinkick(r[k], pl, K2);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) fastdrift<kFast>(r[k], nl2[k], c2[k]);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
+            }
+#pragma unroll
+            for (int k = 0; k < NP; ++k) fastdrift<kFast>(r[k], nl1[k], c1[k]);
+        }
+    }
+}
+
+/* The integration steps with the coefficients of MaxOrder MO in registers
+ * (-1: read from the table on every kick). */
+template <int NP, int MO, bool BEND, bool RAD, bool SKEW>
+__device__ __forceinline__ void multipole_steps_mo(P6* r, Recip* c, const Rec& e, const Param& pm,
+                                                   const double* dp0, const double* nl1,
+                                                   const double* nl2, double irho, int ns) {
+    const int mo = e.mo();
+    const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
+    Poly<MO, SKEW> pl;
+    pl.load(A, A + mo + 1, mo);
+    if (pm.k >= 0) pl.set_param(pm.k, pm.v);
+    if constexpr (kFast) multipole_steps_fast<NP, BEND, RAD>(r, c, e, pl, nl1, nl2, irho, ns);
+    else multipole_steps_rn<NP, BEND, RAD>(r, c, e, pl, pm, dp0, nl1, nl2, irho, ns);
+}
+
+template <int NP, bool BEND, bool RAD, bool GEN, class T>
+__device__ __forceinline__ void multipole_steps(P6T<T>* r, RecipOf<T>* c, const Rec& e,
+                                                const Param& pm, const double* dp0, const T* nl1,
+                                                const T* nl2, double irho, int ns) {
+    if constexpr (is_dual<T>::value) {
+        /* one generic instance for the tangent kernel keeps its size sane */
+        const int mo = e.mo();
+        const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
+        Poly<-1> pl;
+        pl.load(A, A + mo + 1, mo);
+        if (pm.k >= 0) pl.set_param(pm.k, pm.v);
+        multipole_steps_plain<NP, BEND, RAD>(r, e, pl, nl1, nl2, irho, ns);
+    } else {
+        /* tables compiled for another integrator of the GPU call take one
+           generic instance, in the kernels built with them (GEN); the hosts
+           of the other kernels send them none (atb_track_noalloc checks its
+           raw table with a scan kernel, the tangent host refuses it) */
+        if constexpr (GEN) {
+            if (e.flags() & ATB_F_INTEG) {
+                const int mo = e.mo();
+                const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
+                Poly<-1> pl;
+                pl.load(A, A + mo + 1, mo);
+                if (pm.k >= 0) pl.set_param(pm.k, pm.v);
+                /* steps of SL*c[i] drift and SL*d[i] kick
+                   (atgpu/SymplecticIntegrator.cpp:140-171) */
+                multipole_steps_generic<NP, BEND, RAD>(r, e, pl, nl2, irho, ns);
+                return;
+            }
+        }
+#define ATB_STEPS(MO, SKEW) \
+    multipole_steps_mo<NP, MO, BEND, RAD, SKEW>(r, c, e, pm, dp0, nl1, nl2, irho, ns)
+        /* upright magnets' fields without the zero skew terms */
+        const bool upright = e.flags() & ATB_F_NOSKEW;
+        switch (e.mo()) {
+            case 0: ATB_STEPS(0, true); break;
+            case 1:
+                if (upright) ATB_STEPS(1, false);
+                else ATB_STEPS(1, true);
+                break;
+            case 2:
+                if (upright) ATB_STEPS(2, false);
+                else ATB_STEPS(2, true);
+                break;
+            case 3:
+                if (upright) ATB_STEPS(3, false);
+                else ATB_STEPS(3, true);
+                break;
+            default: ATB_STEPS(-1, true); break;
+        }
+#undef ATB_STEPS
+    }
 }
 
 /* StrMPoleSymplectic4Pass.c:29-109, BndMPoleSymplectic4Pass.c:38-129,
  * StrMPoleSymplectic4RadPass.c:30-115, BndMPoleSymplectic4RadPass.c:39-128.
  * NP particles of one thread pass the element together: every per-particle
- * step is an unrolled loop over them, so in the slice loop their drifts and
+ * step is an unrolled loop over them, so in the step loop their drifts and
  * kicks form one straight-line block whose independent chains the compiler
  * interleaves (NP = 2), while the element's parameters are read once.  Each
- * particle sees the same operations as alone (NP = 1). */
-template <int NP, int MO, bool BEND, bool RAD, bool SKEW = true, bool GEN = false, class T>
-__device__ __forceinline__ void pass_multipole_n(P6T<T>* r, const Rec& e, const Param& pm) {
+ * particle sees the same operations as alone (NP = 1).  The entrance and exit
+ * are outside the choice of the step loop: one copy per pass method, which a
+ * warp walking the lattice finds in the instruction cache. */
+template <int NP, bool BEND, bool RAD, bool GEN = false, class T>
+__device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const Rec& e,
+                                                 const Param& pm) {
     const uint32_t fl = e.flags();
-    const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2);
-    const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
-    const int mo = e.mo();
-    const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
-    const double* B = A + mo + 1;
-    Poly<MO, SKEW> pl;
-    pl.load(A, B, mo);
-    if (pm.k >= 0) pl.set_param(pm.k, pm.v);
-
-    T pn0[NP], dp0[NP], nl1[NP], nl2[NP];
+    double dp0[NP];
+    T nl1[NP], nl2[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         if (fl & ATB_F_SCALING) change_pref<kFast>(r[k], e.f(ATB_SM_SCALE));
-        pn0[k] = 0.0;
-        dp0[k] = r[k].dp;
+        dp0[k] = val(r[k].dp);
         nl1[k] = 0.0;
         nl2[k] = 0.0;
         if (!RAD) {
-            T p_norm = 1.0 / (1.0 + r[k].dp);
-            pn0[k] = p_norm;
-            nl1[k] = L1 * p_norm;
-            nl2[k] = L2 * p_norm;
+            T p_norm = opd_rcp(c[k], r[k].dp);
+            nl1[k] = e.f(ATB_SM_L1) * p_norm;
+            nl2[k] = e.f(ATB_SM_L2) * p_norm;
         }
-        entrance_misalign(r[k], e);
-        apertures(r[k], e);
+        if (e.opt) {
+            entrance_misalign(r[k], e);
+            apertures(r[k], e);
+        }
     }
-    double irho = 0.0, k1i = 0.0, k2i = 0.0;
+    double irho = 0.0;
     if (BEND) {
         irho = e.f(ATB_BM_IRHO);
-        k1i = e.f(ATB_BM_K1IRHO);
-        k2i = e.f(ATB_BM_K2IRHO);
         const int m_in = (int)((fl >> ATB_F_BM_IN_SHIFT) & ATB_F_BM_MASK);
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
@@ -492,94 +698,7 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, const Rec& e, const 
             }
         }
     }
-    const int ns = e.nsteps();
-    if constexpr (GEN) {
-        /* another integrator of the GPU call: steps of SL*c[i] drift and
-           SL*d[i] kick (atgpu/SymplecticIntegrator.cpp:140-171) */
-        multipole_steps_generic<NP, BEND, RAD>(r, e, pl, nl2, irho, ns);
-    } else if constexpr (is_dual<T>::value) {
-        multipole_steps_plain<NP, BEND, RAD>(r, e, pl, nl1, nl2, irho, ns);
-    } else if constexpr (!kFast) {
-        multipole_steps_rn<NP, BEND, RAD>(r, e, pl, pm, pn0, dp0, nl1, nl2, irho, ns);
-    } else if (RAD) {
-        const double radc = e.f(ATB_SM_RADC);
-        if constexpr (kFast && !is_dual<T>::value) {
-            if (ns > 0) {
-                const double rk1 = radc * K1, rk2 = radc * K2;
-                const double h1 = 0.5 * L1, h2 = 0.5 * L2;
-                RadAngles a[NP];
-#pragma unroll
-                for (int k = 0; k < NP; ++k) {
-                    const double pn = 1.0 / (1.0 + r[k].dp);
-                    a[k] = RadAngles{r[k].px * pn, r[k].py * pn, 0.0, 1.0 + r[k].dp};
-                }
-                for (int m = 0; m < ns; ++m) {
-#pragma unroll
-                    for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L1, h1);
-#pragma unroll
-                    for (int k = 0; k < NP; ++k) {
-                        if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K1, irho, k1i, rk1);
-                        else str_kick_rad_fast(r[k], a[k], pl, K1, rk1);
-                    }
-#pragma unroll
-                    for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L2, h2);
-#pragma unroll
-                    for (int k = 0; k < NP; ++k) {
-                        if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K2, irho, k2i, rk2);
-                        else str_kick_rad_fast(r[k], a[k], pl, K2, rk2);
-                    }
-#pragma unroll
-                    for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L2, h2);
-#pragma unroll
-                    for (int k = 0; k < NP; ++k) {
-                        if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K1, irho, k1i, rk1);
-                        else str_kick_rad_fast(r[k], a[k], pl, K1, rk1);
-                    }
-#pragma unroll
-                    for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L1, h1);
-                }
-#pragma unroll
-                for (int k = 0; k < NP; ++k) {
-                    r[k].px = a[k].xp * a[k].opd;
-                    r[k].py = a[k].yp * a[k].opd;
-                }
-            }
-        }
-    } else {
-        T c1[NP], c2[NP];
-#pragma unroll
-        for (int k = 0; k < NP; ++k) {
-            c1[k] = 0.0;
-            c2[k] = 0.0;
-            if (kFast) {
-                T h = 0.5 / (1.0 + r[k].dp);
-                c1[k] = nl1[k] * h;
-                c2[k] = nl2[k] * h;
-            }
-        }
-        for (int m = 0; m < ns; ++m) {
-#pragma unroll
-            for (int k = 0; k < NP; ++k) fastdrift<kFast>(r[k], nl1[k], c1[k]);
-#pragma unroll
-            for (int k = 0; k < NP; ++k) {
-                if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
-            }
-#pragma unroll
-            for (int k = 0; k < NP; ++k) fastdrift<kFast>(r[k], nl2[k], c2[k]);
-#pragma unroll
-            for (int k = 0; k < NP; ++k) {
-                if (BEND) bndthinkick(r[k], pl, K2, irho, k2i); else strthinkick(r[k], pl, K2);
-            }
-#pragma unroll
-            for (int k = 0; k < NP; ++k) fastdrift<kFast>(r[k], nl2[k], c2[k]);
-#pragma unroll
-            for (int k = 0; k < NP; ++k) {
-                if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
-            }
-#pragma unroll
-            for (int k = 0; k < NP; ++k) fastdrift<kFast>(r[k], nl1[k], c1[k]);
-        }
-    }
+    multipole_steps<NP, BEND, RAD, GEN>(r, c, e, pm, dp0, nl1, nl2, irho, e.nsteps());
     if (fl & ATB_F_FQ_OUT) {
         const T b1 = fringe_b1<T>(e, pm);
 #pragma unroll
@@ -607,63 +726,26 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, const Rec& e, const 
                                    e.f(ATB_BM_FXOUT), e.f(ATB_BM_FYOUT), m_out,
                                    fl & ATB_F_FC0_OUT, -1.0);
         }
-        apertures(r[k], e);
-        exit_misalign(r[k], e);
+        if (e.opt) {
+            apertures(r[k], e);
+            exit_misalign(r[k], e);
+        }
         if (fl & ATB_F_SCALING) change_pref<kFast>(r[k], e.f(ATB_SM_ISCALE));
     }
 }
 
-template <int NP, bool BEND, bool RAD, bool GEN = false, class T>
-__device__ __forceinline__ void pass_multipole_dispatch_n(P6T<T>* r, const Rec& e,
-                                                          const Param& pm) {
-    if constexpr (is_dual<T>::value) {
-        /* one generic instance for the tangent kernel keeps its size sane */
-        pass_multipole_n<NP, -1, BEND, RAD>(r, e, pm);
-    } else {
-        /* tables compiled for another integrator of the GPU call take one
-           generic instance, in the kernels built with them (GEN); the hosts
-           of the other kernels send them none (atb_track_noalloc checks its
-           raw table with a scan kernel, the tangent host refuses it) */
-        if constexpr (GEN) {
-            if (e.flags() & ATB_F_INTEG) {
-                pass_multipole_n<NP, -1, BEND, RAD, true, true>(r, e, pm);
-                return;
-            }
-        }
-        /* upright magnets' fields without the zero skew terms */
-        const bool upright = e.flags() & ATB_F_NOSKEW;
-        switch (e.mo()) {
-            case 0: pass_multipole_n<NP, 0, BEND, RAD>(r, e, pm); break;
-            case 1:
-                if (upright) pass_multipole_n<NP, 1, BEND, RAD, false>(r, e, pm);
-                else pass_multipole_n<NP, 1, BEND, RAD>(r, e, pm);
-                break;
-            case 2:
-                if (upright) pass_multipole_n<NP, 2, BEND, RAD, false>(r, e, pm);
-                else pass_multipole_n<NP, 2, BEND, RAD>(r, e, pm);
-                break;
-            case 3:
-                if (upright) pass_multipole_n<NP, 3, BEND, RAD, false>(r, e, pm);
-                else pass_multipole_n<NP, 3, BEND, RAD>(r, e, pm);
-                break;
-            default: pass_multipole_n<NP, -1, BEND, RAD>(r, e, pm); break;
-        }
-    }
-}
-
-template <bool BEND, bool RAD, bool GEN = false, class T>
-__device__ __forceinline__ void pass_multipole_dispatch(P6T<T>& r, const Rec& e, const Param& pm) {
-    pass_multipole_dispatch_n<1, BEND, RAD, GEN>(&r, e, pm);
-}
-
 /* DriftPass.c:16-48 */
 template <class T>
-__device__ __forceinline__ void pass_drift(P6T<T>& r, const Rec& e) {
-    entrance_misalign(r, e);
-    apertures(r, e);
-    drift6<kFast>(r, e.f(ATB_DR_LE));
-    apertures(r, e);
-    exit_misalign(r, e);
+__device__ __forceinline__ void pass_drift(P6T<T>& r, RecipOf<T>& c, const Rec& e) {
+    if (e.opt) {
+        entrance_misalign(r, e);
+        apertures(r, e);
+    }
+    drift6_pn<kFast>(r, e.f(ATB_DR_LE), opd_rcp(c, r.dp));
+    if (e.opt) {
+        apertures(r, e);
+        exit_misalign(r, e);
+    }
 }
 
 /* IdentityPass.c:20-43 */
@@ -763,18 +845,18 @@ __device__ __forceinline__ void pass_quantdiff(P6T<T>& r, const Rec& e, const At
 }
 
 template <bool GEN = false, class T>
-__device__ __forceinline__ void track_element(P6T<T>& r, const Rec& e, int nturn,
+__device__ __forceinline__ void track_element(P6T<T>& r, RecipOf<T>& c, const Rec& e, int nturn,
                                               const Param& pm = Param{-1, 0.0},
                                               const AtbRng* rng = nullptr, long long p = 0,
                                               int ei = 0) {
     if (isnan(val(r.x))) return;
     switch (e.op()) {
         case ATB_OP_IDENTITY: pass_identity(r, e); break;
-        case ATB_OP_DRIFT: pass_drift(r, e); break;
-        case ATB_OP_STRMPOLE: pass_multipole_dispatch<false, false, GEN>(r, e, pm); break;
-        case ATB_OP_STRMPOLE_RAD: pass_multipole_dispatch<false, true, GEN>(r, e, pm); break;
-        case ATB_OP_BNDMPOLE: pass_multipole_dispatch<true, false, GEN>(r, e, pm); break;
-        case ATB_OP_BNDMPOLE_RAD: pass_multipole_dispatch<true, true, GEN>(r, e, pm); break;
+        case ATB_OP_DRIFT: pass_drift(r, c, e); break;
+        case ATB_OP_STRMPOLE: pass_multipole_n<1, false, false, GEN>(&r, &c, e, pm); break;
+        case ATB_OP_STRMPOLE_RAD: pass_multipole_n<1, false, true, GEN>(&r, &c, e, pm); break;
+        case ATB_OP_BNDMPOLE: pass_multipole_n<1, true, false, GEN>(&r, &c, e, pm); break;
+        case ATB_OP_BNDMPOLE_RAD: pass_multipole_n<1, true, true, GEN>(&r, &c, e, pm); break;
         case ATB_OP_THINMPOLE: pass_thinmpole(r, e, pm); break;
         case ATB_OP_RFCAVITY: pass_rfcavity(r, e, nturn); break;
         case ATB_OP_CORRECTOR: pass_corrector(r, e); break;
@@ -799,13 +881,14 @@ __device__ __forceinline__ bool track_together(const P6 (&r)[NP], const Rec& e) 
 }
 
 template <int NP>
-__device__ __forceinline__ void pass_multipoles_together(P6 (&r)[NP], const Rec& e) {
+__device__ __forceinline__ void pass_multipoles_together(P6 (&r)[NP], Recip (&c)[NP],
+                                                         const Rec& e) {
     const Param none{-1, 0.0};
     switch (e.op()) {
-        case ATB_OP_STRMPOLE: pass_multipole_dispatch_n<NP, false, false>(r, e, none); break;
-        case ATB_OP_STRMPOLE_RAD: pass_multipole_dispatch_n<NP, false, true>(r, e, none); break;
-        case ATB_OP_BNDMPOLE: pass_multipole_dispatch_n<NP, true, false>(r, e, none); break;
-        default: pass_multipole_dispatch_n<NP, true, true>(r, e, none); break;
+        case ATB_OP_STRMPOLE: pass_multipole_n<NP, false, false>(r, c, e, none); break;
+        case ATB_OP_STRMPOLE_RAD: pass_multipole_n<NP, false, true>(r, c, e, none); break;
+        case ATB_OP_BNDMPOLE: pass_multipole_n<NP, true, false>(r, c, e, none); break;
+        default: pass_multipole_n<NP, true, true>(r, c, e, none); break;
     }
 }
 
@@ -945,22 +1028,12 @@ __device__ __forceinline__ bool serve_requeue(const AtbServeRing& ring, const At
 
 #if ATB_KERNELS
 
-/* lost-particle marking of one particle after an element (pyat/at.c:115-161) */
-__device__ __forceinline__ void apply_loss_rule(const AtbJob& J, P6& r, bool& lost, bool active,
-                                                long long p, int nturn, int ei) {
-    if (J.losses) {
-        if (!lost && is_bad(r)) {
-            lost = true;
-            if (active) {
-                J.lturn[p] = (unsigned)nturn;
-                J.lelem[p] = (unsigned)ei;
-                store6(J.lcoord + 6 * p, r);
-            }
-            r.x = nan_d(); r.px = 0.0; r.y = 0.0; r.py = 0.0; r.dp = 0.0; r.ct = 0.0;
-        }
-    } else if (isfinite(r.x) && is_bad(r)) {
-        r.x = nan_d(); r.px = 0.0; r.y = 0.0; r.py = 0.0; r.dp = 0.0; r.ct = 0.0;
-    }
+/* the loss map of one particle, written once (pyat/at.c:115-161) */
+__device__ __forceinline__ void record_loss(const AtbJob& J, const P6& r, long long p, int nturn,
+                                            int ei) {
+    J.lturn[p] = (unsigned)nturn;
+    J.lelem[p] = (unsigned)ei;
+    store6(J.lcoord + 6 * p, r);
 }
 
 /* The persistent tile loop.  NP particles per thread: particle k of thread t
@@ -1080,7 +1153,12 @@ __device__ __forceinline__ void track_tiles(const AtbJob* __restrict__ jobs,
         bool exhausted = false;         /* the job cursor has no particle left */
         const bool resident = (J.resident != 0);
 
+        /* read once: a store to global memory would have the element loop
+           read them from the job again */
+        const bool check_loss = J.check_loss != 0, losses = J.losses != 0;
+
         P6 r[NP];
+        Recip rc[NP];
         bool lost[NP];
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
@@ -1188,17 +1266,25 @@ __device__ __forceinline__ void track_tiles(const AtbJob* __restrict__ jobs,
                     bool together = false;
                     if constexpr (NP > 1) together = track_together(r, e);
                     if (together) {
-                        if constexpr (NP > 1) pass_multipoles_together(r, e);
+                        if constexpr (NP > 1) pass_multipoles_together(r, rc, e);
                     } else {
 #pragma unroll
                         for (int k = 0; k < NP; ++k)
-                            track_element<GEN>(r[k], e, nturn[k], Param{-1, 0.0}, &J.rng,
+                            track_element<GEN>(r[k], rc[k], e, nturn[k], Param{-1, 0.0}, &J.rng,
                                                p[k], ei);
                     }
+                    if (check_loss) {
 #pragma unroll
-                    for (int k = 0; k < NP; ++k)
-                        if (J.check_loss)
-                            apply_loss_rule(J, r[k], lost[k], active[k], p[k], nturn[k], ei);
+                        for (int k = 0; k < NP; ++k)
+                            if (losses ? !lost[k] && is_bad(r[k])
+                                       : isfinite(r[k].x) && is_bad(r[k])) {
+                                if (losses && active[k])
+                                    record_loss(J, r[k], p[k], nturn[k], ei);
+                                lost[k] = true;
+                                r[k].x = nan_d(); r[k].px = 0.0; r[k].y = 0.0;
+                                r[k].py = 0.0; r[k].dp = 0.0; r[k].ct = 0.0;
+                            }
+                    }
                     w += e.len();
                 }
                 if (!resident) {

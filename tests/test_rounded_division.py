@@ -27,10 +27,16 @@ void step_(long n, const double* d, const double* y, double* q)
 void from_(long n, const double* o, const double* s, double* q, int* ok)
 { for (long i = 0; i < n; ++i) { double e; q[i] = rn_rcp_from(o[i], s[i], &e);
     ok[i] = rn_below(e, ATB_RN_SEED_HI) && rn_opd_fits(o[i]) && !rn_below_one(o[i]); } }
+void nearer_(long n, const double* d, double* q, int* ok)
+{ for (long i = 0; i < n; ++i) { q[i] = rn_rcp_nearer(d[i]); ok[i] = rn_nearer_fits(d[i]); } }
 void near_(long n, const double* d, double* q, int* ok)
 { for (long i = 0; i < n; ++i) { q[i] = rn_rcp_near(d[i]); ok[i] = rn_near_fits(d[i]); } }
-void fit_(long n, const double* a, int* ok)
-{ for (long i = 0; i < n; ++i) ok[i] = rn_fit(a[i]); }
+#define TEST_FN(name, f) void name(long n, const double* a, int* ok) \
+{ for (long i = 0; i < n; ++i) ok[i] = f(a[i]); }
+TEST_FN(coord_, rn_coord_fits)
+TEST_FN(length_, rn_length_fits)
+TEST_FN(square_, rn_square_fits)
+TEST_FN(tiny_, rn_not_tiny)
 """
 
 
@@ -43,16 +49,18 @@ def rn(tmp_path_factory):
                     "-I", os.path.join(ROOT, "at_b200", "csrc"), "-lm"], check=True)
     lib = C.CDLL(str(so))
 
-    def call(name, *arrays, flags=False):
+    def call(name, *arrays, flags=False, test=False):
         n = arrays[0].size
         args = [np.ascontiguousarray(a, dtype=np.float64) for a in arrays]
         out, ok = np.empty(n), np.empty(n, dtype=np.int32)
         ptrs = [a.ctypes.data_as(C.c_void_p) for a in args]
-        if name != "fit_":
+        if not test:
             ptrs.append(out.ctypes.data_as(C.c_void_p))
         if flags:
             ptrs.append(ok.ctypes.data_as(C.c_void_p))
         getattr(lib, name)(C.c_long(n), *ptrs)
+        if test:
+            return ok.astype(bool)
         return (out, ok.astype(bool)) if flags else out
     return call
 
@@ -103,6 +111,10 @@ def test_reciprocals_equal_ieee_division(rn):
     q, ok = rn("near_", d, flags=True)
     assert ok.mean() > 0.9
     np.testing.assert_array_equal(q[ok], 1.0 / d[ok])
+    d = 1.0 + rng.uniform(0, 1, n) * np.ldexp(1.0, -rng.integers(9, 53, n))
+    q, ok = rn("nearer_", d, flags=True)
+    assert ok.mean() > 0.9
+    np.testing.assert_array_equal(q[ok], 1.0 / d[ok])
     seed = 1.0 / _near_one(rng, n, 0.125)
     o = (1.0 / seed) * (1.0 + rng.uniform(-1, 1, n) * np.ldexp(1.0, -rng.integers(19, 54, n)))
     q, ok = rn("from_", o, seed, flags=True)
@@ -110,12 +122,20 @@ def test_reciprocals_equal_ieee_division(rn):
     np.testing.assert_array_equal(q[ok], 1.0 / o[ok])
 
 
-def test_accepted_numerators(rn):
-    a = np.array([0.0, -0.0, 1.0, -1.0, 2.0 ** -900, 2.0 ** -901, 5e-324, -5e-324, 2.0 ** 899,
-                  2.0 ** 900, np.inf, -np.inf, np.nan])
-    _, ok = rn("fit_", a, flags=True)
-    assert ok.tolist() == [True, True, True, True, True, False, False, False, True, False, False,
-                           False, False]
+def test_accepted_operands(rn):
+    """Each test's bounds; zeros pass, nothing else that is tiny does."""
+    for name, low, high in (("coord_", -400, 900), ("length_", -40, 40), ("square_", -860, None),
+                            ("tiny_", -480, None)):
+        lo = 2.0 ** low
+        a = np.array([0.0, 1.0, lo, np.nextafter(lo, 0.0), 2.0 ** -1040])
+        ok = [True, True, True, False, False]
+        if name != "square_":                       # the others take either sign
+            a, ok = np.concatenate((a, -a)), ok + ok
+        if high is not None:                        # exact to the last denormal, bounded above
+            hi = 2.0 ** high
+            a = np.concatenate((a, [5e-324, np.nextafter(hi, 0.0), hi, np.inf, -np.inf, np.nan]))
+            ok = ok + [False, True, False, False, False, False]
+        assert rn(name, a, flags=True, test=True).tolist() == ok, name
 
 
 # -- on the GPU -----------------------------------------------------------------
@@ -129,7 +149,7 @@ def _edge_particles():
     base[0:2, 24:40] = 0.0
     base[4, 40:72] = np.linspace(-0.13, 0.13, 32)            # 1 + delta around 7/8 and 9/8
     base[4, 72:80] = [2.0 ** -53, -2.0 ** -53, -2.0 ** -54, 2.0 ** -52, 1e-300, -1e-16, 0.0, -0.0]
-    base[3, 80:96] = np.ldexp(1.0, -np.linspace(860, 1074, 16).astype(int))   # tiny angles
+    base[3, 80:96] = np.ldexp(1.0, -np.linspace(390, 1074, 16).astype(int))   # tiny angles
     base[1, 88:96] = 0.0
     base[0, 96:112] = np.linspace(0.05, 0.9, 16)             # far from the axis
     base[1, 112:128] = np.linspace(0.01, 0.5, 16)            # steep
