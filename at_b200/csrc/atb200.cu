@@ -160,6 +160,7 @@ struct atb_handle {
     std::vector<int32_t> h_pelem;
     std::vector<AtbTile> h_tiles;
     std::vector<struct Batch> batches;
+    cudaEvent_t launched = nullptr;    /* the last launch that uses the handle's lists */
     char* stage[2] = {nullptr, nullptr};            /* pinned snapshot staging */
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};
 };
@@ -340,6 +341,18 @@ int launch(atb_handle* h, const std::vector<AtbJob>& jobs, const std::vector<Atb
            int smem_bytes, int grid_max, int mode, cudaStream_t st, int threads, int ppt,
            bool gen) {
     if (tiles.empty()) return ATB_OK;
+    /* The launch lists, counters and scratch belong to the handle: a launch on
+       another stream waits for the last one before it replaces them.  (Inside
+       a stream capture there is nothing to wait for or to record.) */
+    cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
+    ATB_CUDA(cudaStreamIsCapturing(st, &cap_st));
+    const bool ordered = cap_st == cudaStreamCaptureStatusNone;
+    if (ordered) {
+        if (!h->launched)
+            ATB_CUDA(cudaEventCreateWithFlags(&h->launched, cudaEventDisableTiming));
+        else
+            ATB_CUDA(cudaStreamWaitEvent(st, h->launched, 0));
+    }
     if (h->jobs.ensure(jobs.size() * sizeof(AtbJob)) != cudaSuccess ||
         h->tiles.ensure(tiles.size() * sizeof(AtbTile)) != cudaSuccess)
         return fail(ATB_ERR_CUDA, "cudaMalloc(launch lists) failed");
@@ -384,6 +397,7 @@ int launch(atb_handle* h, const std::vector<AtbJob>& jobs, const std::vector<Atb
         atb_track_kernel_fast<<<grid, threads, smem_bytes, st>>>(dj, dt, nt, cnt, jn, sts, cap,
                                                                  scr);
     ATB_CUDA(cudaGetLastError());
+    if (ordered) ATB_CUDA(cudaEventRecord(h->launched, st));
     return ATB_OK;
 }
 
@@ -577,6 +591,7 @@ int atb_destroy(atb_handle* h) {
             if (h->stage[i]) cudaFreeHost(h->stage[i]);
             if (h->stage_ev[i]) cudaEventDestroy(h->stage_ev[i]);
         }
+        if (h->launched) cudaEventDestroy(h->launched);
         if (h->stream) cudaStreamDestroy(h->stream);
     }
     delete h;
