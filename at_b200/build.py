@@ -28,11 +28,12 @@ UNITS = [
       for arith, fmad in (("exact", "false"), ("fast", "true"))
       for kern in ("BASE", "GEN", "SERVE", "NP2")],
     ("tangent", "tangent.cu", ["-fmad=false"]),
+    ("tangent_plain", "tangent_plain.cu", ["-fmad=false"]),
     ("adjoint", "adjoint.cu", ["-fmad=false"]),
     ("atb200", "atb200.cu", []),
     ("atb_noalloc", "atb_noalloc.cu", []),
 ]
-DEPS = ["atb_physics.cuh", "atb_dual.cuh", "track_kernel.cuh", "tangent_kernel.cuh",
+DEPS = ["atb_physics.cuh", "atb_dual.cuh", "track_kernel.cuh", "tangent_kernel.cuh", "tangent_plain.cuh", "atb_solve6.cuh",
         "adjoint_kernel.cuh",
         "atb_diffusion.cuh", "atb_integrators.h", "atb_rn.h",
         "atb_kernel_api.h", "atb_table.h"]

@@ -65,6 +65,7 @@ extern "C" __global__ void atb_serve_kernel_exact(const AtbJob*, const AtbTile*,
 extern "C" __global__ void atb_serve_kernel_fast(const AtbJob*, const AtbTile*, AtbServeArgs, int*,
                                                  int*, int, double*);
 extern "C" __global__ void atb_tangent_kernel(const AtbTangent);
+extern "C" __global__ void atb_tangent_plain_kernel(const AtbTangent);
 extern "C" __global__ void atb_adjoint_forward_kernel(const AtbAdjoint);
 extern "C" __global__ void atb_adjoint_turn_kernel(const AtbAdjoint);
 extern "C" __global__ void atb_element_maps_kernel(const AtbElemMaps);
@@ -1097,6 +1098,15 @@ int strength_map(atb_handle* h, const Lattice* L, const int32_t* param_elem,
     return ATB_OK;
 }
 
+static bool tangent_by_hand(const Lattice& L) {
+    for (const uint64_t hdr : L.hdr) {
+        const uint32_t op = (uint32_t)((hdr >> ATB_H_OP_SHIFT) & ATB_H_OP_MASK);
+        const uint32_t fl = (uint32_t)((hdr >> ATB_H_FL_SHIFT) & ATB_H_FL_MASK);
+        if (!atb_tangent_by_hand(op, fl)) return false;
+    }
+    return true;
+}
+
 int atb_tangent_device(atb_handle* h, int32_t id, double* r, int64_t np, int32_t nturns,
                        int32_t turn0, const int32_t* param_elem, const int32_t* param_order,
                        const double* param_value, int32_t nparam, double* jac, double* grad,
@@ -1141,7 +1151,10 @@ int atb_tangent_device(atb_handle* h, int32_t id, double* r, int64_t np, int32_t
     A.lost = islost;
     const long long blocks = (np + ATB_TANGENT_THREADS - 1) / ATB_TANGENT_THREADS;
     if (blocks > 0x7fffffffLL) return fail(ATB_ERR_ARG, "too many particles");
-    atb_tangent_kernel<<<(unsigned)blocks, ATB_TANGENT_THREADS, 0, st>>>(A);
+    if (tangent_by_hand(*L))
+        atb_tangent_plain_kernel<<<(unsigned)blocks, ATB_TANGENT_THREADS, 0, st>>>(A);
+    else
+        atb_tangent_kernel<<<(unsigned)blocks, ATB_TANGENT_THREADS, 0, st>>>(A);
     ATB_CUDA(cudaGetLastError());
     return ATB_OK;
 }

@@ -28,6 +28,7 @@
 #define ATB_TANGENT_KERNEL_CUH
 
 #include "track_kernel.cuh"
+#include "atb_solve6.cuh"
 
 namespace atb {
 
@@ -37,9 +38,7 @@ using TD = Dual<kTanDirs>;
 /* rows of the state as an array of dual numbers (compile-time indices only) */
 #define ATB_ROWS(r) {&(r).x, &(r).px, &(r).y, &(r).py, &(r).dp, &(r).ct}
 
-/* w = J^-1 g for J[i][j] = row_i.d[j], g_i = row_i.d[6]: Gaussian elimination
- * with partial pivoting on a 6x7 augmented matrix held in registers (row
- * swaps are selects, so every index is known at compile time). */
+/* w = J^-1 g for J[i][j] = row_i.d[j], g_i = row_i.d[6] */
 __device__ __forceinline__ void solve_tangent(P6T<TD>& r, double w[6]) {
     TD* rows[6] = ATB_ROWS(r);
     double M[6][7];
@@ -48,41 +47,7 @@ __device__ __forceinline__ void solve_tangent(P6T<TD>& r, double w[6]) {
 #pragma unroll
         for (int j = 0; j < 7; ++j) M[i][j] = rows[i]->d[j];
     }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        /* pivot: the largest |M[i][c]|, i >= c */
-        double best = fabs(M[c][c]);
-        int piv = c;
-#pragma unroll
-        for (int i = c + 1; i < 6; ++i) {
-            const double a = fabs(M[i][c]);
-            if (a > best) { best = a; piv = i; }
-        }
-#pragma unroll
-        for (int i = c + 1; i < 6; ++i) {
-            const bool sw = (piv == i);
-#pragma unroll
-            for (int j = c; j < 7; ++j) {
-                const double t = M[c][j];
-                M[c][j] = sw ? M[i][j] : t;
-                M[i][j] = sw ? t : M[i][j];
-            }
-        }
-        const double inv = 1.0 / M[c][c];
-#pragma unroll
-        for (int i = c + 1; i < 6; ++i) {
-            const double f = M[i][c] * inv;
-#pragma unroll
-            for (int j = c + 1; j < 7; ++j) M[i][j] -= f * M[c][j];
-        }
-    }
-#pragma unroll
-    for (int i = 5; i >= 0; --i) {
-        double s = M[i][6];
-#pragma unroll
-        for (int j = i + 1; j < 6; ++j) s -= M[i][j] * w[j];
-        w[i] = s / M[i][i];
-    }
+    solve6(M, w);
 }
 
 extern "C" __global__ void __launch_bounds__(ATB_TANGENT_THREADS)
