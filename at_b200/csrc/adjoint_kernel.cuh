@@ -13,12 +13,12 @@
  * of this unit ("exact" arithmetic, so the values equal the exact tracking
  * kernel's), and the state entering every stride-th turn is stored.
  *
- * Backward (atb_adjoint_turn_kernel, one launch per turn, last turn first):
- * from the turn's entry state the turn is tracked again, every element's
- * entry state going to a scratch array ([element][particle][6], coalesced)
- * -- or, when the forward pass stored every turn's element-entry states
- * (memory permitting), those are read instead;
- * then the elements are walked backwards with lambda <- J_e^T lambda, J_e
+ * Backward (two launches per turn, last turn first): the forward kernel
+ * tracks the turn again from its entry state, every element's entry state
+ * going to a scratch array ([element][particle][6], coalesced) -- or the
+ * forward pass stored every turn's (memory permitting); then
+ * atb_adjoint_turn_kernel walks the elements backwards with
+ * lambda <- J_e^T lambda, J_e
  * the element's Jacobian at its stored entry state, and at an element that
  * carries K_q, dL/dK_q += (d r_out / d K_q) . lambda_out, summed over the
  * block's particles in shared memory and added to the global sum once per
@@ -28,12 +28,10 @@
  *  - DriftPass, IdentityPass, AperturePass, RFCavityPass, thin
  *    CorrectorPass, ThinMPolePass and the non-radiating StrMPole/BndMPole
  *    Symplectic4 passes (plain or bend-edge entrance/exit, misaligned or
- *    not): written out by hand.  In a thick magnet the
- *    (x, px, y, py) entering each integration step are recomputed from the
- *    element's entry state into a per-thread store in shared memory (every step up to
- *    ATB_ADJ_STEPS steps, every ceil(n / ATB_ADJ_STEPS)-th beyond, the rest
- *    recomputed from the nearest), each step is re-run with the inputs of its
- *    seven stages kept in registers, and the stages are reversed: the
+ *    not): written out by hand.  A thick magnet is walked
+ *    backwards from its exit state (the next element's entry state): every
+ *    stage is undone on (x, px, y, py) -- a drift or kick is its own inverse
+ *    but for the sign -- and reversed at the coordinates so found: the
  *    fastdrift (driftkick.c:37-48), and the kick (driftkick.c:51-115) with the
  *    field derivative F'(z) of F(z) = sum (B_n + i A_n) z^n from a second
  *    Horner recursion and dF/dB_k = z^k for the strength.
@@ -43,6 +41,12 @@
  *    line so that its registers do not weigh on the common path.
  * A particle that is lost (NaN, or lost during the turn) gets a NaN
  * cotangent and adds nothing to the strengths' gradient.
+ *
+ * Bound by dependent FP64 latency at 3.5 warps a scheduler (65,536 particles).
+ * A turn of the FODO ring with 128 strengths backwards: 5.0 ms with the step
+ * entries recomputed into shared memory and every step run twice more; 2.4 ms
+ * with the stages undone from the exit (1.0 of it the tracking), which needs
+ * no store and keeps one stage's coordinates instead of seven.
  */
 #ifndef ATB_ADJOINT_KERNEL_CUH
 #define ATB_ADJOINT_KERNEL_CUH
@@ -51,19 +55,6 @@
 
 namespace atb {
 
-/* integration-step entry states kept per thread, in shared memory */
-#define ATB_ADJ_STEPS ATB_ADJ_STEPS_SMEM
-
-/* A thread's step-entry store in the block's shared memory: entry c,
- * component k (x, px, y, py) at base[(4 c + k) * stride], stride the block
- * size, so a warp's accesses fall on consecutive words. */
-struct StepStore {
-    double* base;
-    int stride;
-    __device__ __forceinline__ double& at(int c, int k) const {
-        return base[(4 * c + k) * stride];
-    }
-};
 #ifndef ATB_ADJ_MIN_BLOCKS
 #define ATB_ADJ_MIN_BLOCKS 4   /* 128 registers a thread: the dual-number
                                   fallback spills, the common path does not */
@@ -130,8 +121,7 @@ __device__ __forceinline__ void adj_entrance_misalign(double* lam, const Rec& e)
 
 /* drift6 at input s: x += nl px, y += nl py, ct += nl pn S / 2 with
  * pn = 1/(1+dp), nl = L pn, S = px^2 + py^2 */
-__device__ __forceinline__ void adj_drift6(const P6& s, double* lam, double L) {
-    const double pn = 1.0 / (1.0 + s.dp);
+__device__ __forceinline__ void adj_drift6(const P6& s, double* lam, double L, double pn) {
     const double nl = L * pn;
     const double lx = lam[0], ly = lam[2], lc = lam[5];
     const double S = fma(s.px, s.px, s.py * s.py);
@@ -142,56 +132,86 @@ __device__ __forceinline__ void adj_drift6(const P6& s, double* lam, double L) {
 }
 
 /* DriftPass.c:16-48 */
-__device__ __forceinline__ void adj_pass_drift(const P6& s, double* lam, const Rec& e) {
+__device__ __forceinline__ void adj_pass_drift(const P6& s, Recip& rc, double* lam,
+                                               const Rec& e) {
+    if (!e.opt) {
+        adj_drift6(s, lam, e.f(ATB_DR_LE), opd_rcp(rc, s.dp));
+        return;
+    }
     P6 r = s;
     entrance_misalign(r, e);
     adj_exit_misalign(lam, e);
-    adj_drift6(r, lam, e.f(ATB_DR_LE));
+    adj_drift6(r, lam, e.f(ATB_DR_LE), opd_rcp(rc, r.dp));
     adj_entrance_misalign(lam, e);
 }
 
 /* ---- thick multipoles ---------------------------------------------------- */
 
 /* The element's multipole coefficients for the reverse pass, B_sk replaced
- * by the differentiated strength kv: in registers for MaxOrder MO in 0..3,
- * read from the table for MO = -1 (any order).  field() is F(z) =
- * sum_n (B_n + i A_n) z^n by Horner's rule with fused multiply-adds (the
- * recomputed steps inside an element only feed derivatives, so they need not
- * round as the tracking does); prime() is F'(z) by the same recursion. */
-template <int MO>
+ * by the differentiated strength kv: in registers for MaxOrder MO in 0..3
+ * (SKEW false: every A_n is zero), read from the table for MO = -1 (any
+ * order).  field() is F(z) = sum_n (B_n + i A_n) z^n by Horner's rule with
+ * fused multiply-adds (the recomputed steps inside an element only feed
+ * derivatives, so they need not round as the tracking does); prime() is F'(z)
+ * by the same recursion. */
+template <int MO, bool SKEW>
 struct AdjCoef {
-    double a[MO + 1], b[MO + 1];
+    double a[SKEW ? MO + 1 : 1], b[MO + 1];
     int sk;
     __device__ __forceinline__ void load(const double* A, const double* B, int, int k,
                                          double v) {
 #pragma unroll
         for (int i = 0; i <= MO; ++i) {
-            a[i] = A[i];
+            if (SKEW) a[SKEW ? i : 0] = A[i];
             b[i] = (i == k) ? v : B[i];
         }
         sk = k;
     }
+    __device__ __forceinline__ double an(int i) const { return SKEW ? a[SKEW ? i : 0] : 0.0; }
     __device__ __forceinline__ void field(double x, double y, double& re, double& im) const {
-        re = b[MO];
-        im = a[MO];
+        if constexpr (SKEW || MO == 0) {
+            re = b[MO];
+            im = an(MO);
 #pragma unroll
-        for (int i = MO - 1; i >= 0; --i) {
-            const double t = fma(re, x, fma(-im, y, b[i]));
-            im = fma(im, x, fma(re, y, a[i]));
-            re = t;
+            for (int i = MO - 1; i >= 0; --i) {
+                const double t = fma(re, x, fma(-im, y, b[i]));
+                im = fma(im, x, fma(re, y, an(i)));
+                re = t;
+            }
+        } else {
+            re = fma(b[MO], x, b[MO - 1]);
+            im = b[MO] * y;
+#pragma unroll
+            for (int i = MO - 2; i >= 0; --i) {
+                const double t = fma(re, x, fma(-im, y, b[i]));
+                im = fma(im, x, re * y);
+                re = t;
+            }
         }
     }
     __device__ __forceinline__ void prime(double x, double y, double& dr, double& di) const {
         if constexpr (MO == 0) {
             dr = 0.0;
             di = 0.0;
+        } else if constexpr (!SKEW && MO == 1) {
+            dr = b[1];
+            di = 0.0;
+        } else if constexpr (!SKEW) {
+            dr = fma((double)MO * b[MO], x, (double)(MO - 1) * b[MO - 1]);
+            di = (double)MO * b[MO] * y;
+#pragma unroll
+            for (int n = MO - 2; n >= 1; --n) {
+                const double t = fma(dr, x, fma(-di, y, (double)n * b[n]));
+                di = fma(di, x, dr * y);
+                dr = t;
+            }
         } else {
             dr = (double)MO * b[MO];
-            di = (double)MO * a[MO];
+            di = (double)MO * an(MO);
 #pragma unroll
             for (int n = MO - 1; n >= 1; --n) {
                 const double t = fma(dr, x, fma(-di, y, (double)n * b[n]));
-                di = fma(di, x, fma(dr, y, (double)n * a[n]));
+                di = fma(di, x, fma(dr, y, (double)n * an(n)));
                 dr = t;
             }
         }
@@ -199,7 +219,7 @@ struct AdjCoef {
 };
 
 template <>
-struct AdjCoef<-1> {
+struct AdjCoef<-1, true> {
     const double* a;
     const double* b;
     int mo;
@@ -249,20 +269,22 @@ __device__ __forceinline__ void zpow(double x, double y, int k, double& zr, doub
 /* strthinkick / bndthinkick of length L at input (x, y):
  * px -= L (Re F - [bend] (dp - x irho) irho), py += L Im F,
  * [bend] ct += lirho x */
-template <bool BEND, int MO>
-__device__ __forceinline__ void adj_kick(const AdjCoef<MO>& c, double x, double y, double L,
-                                         double lirho, double irho, double* lam, double& g) {
+template <bool BEND, class C>
+__device__ __forceinline__ void adj_kick(const C& c, double x, double y, double L, double lirho,
+                                         double irho, double* lam, double& g) {
     double dr, di;
     c.prime(x, y, dr, di);
     const double lpx = lam[1], lpy = lam[3];
-    double ax = L * fma(-dr, lpx, di * lpy);
-    const double ay = L * fma(di, lpx, dr * lpy);
+    const double ay = L * dr, b = L * di;
     if (BEND) {
-        ax = fma(-L * irho * irho, lpx, fma(lirho, lam[5], ax));
-        lam[4] = fma(L * irho, lpx, lam[4]);
+        const double li = L * irho;
+        lam[0] = fma(-fma(li, irho, ay), lpx, fma(lirho, lam[5], lam[0]));
+        lam[4] = fma(li, lpx, lam[4]);
+    } else {
+        lam[0] = fma(-ay, lpx, lam[0]);
     }
-    lam[0] += ax;
-    lam[2] += ay;
+    lam[0] = fma(b, lpy, lam[0]);
+    lam[2] = fma(ay, lpy, fma(b, lpx, lam[2]));
     if (c.sk >= 0) {
         double zr, zi;
         zpow(x, y, c.sk, zr, zi);
@@ -270,22 +292,55 @@ __device__ __forceinline__ void adj_kick(const AdjCoef<MO>& c, double x, double 
     }
 }
 
+/* the same in an upright magnet up to the quadrupole, where F' = b1 */
+template <bool BEND, int MO>
+__device__ __forceinline__ void adj_kick(const AdjCoef<MO, false>& c, double x, double y, double L,
+                                         double lirho, double irho, double* lam, double& g) {
+    if constexpr (MO == 1) {
+        const double lpx = lam[1], lpy = lam[3];
+        const double ay = L * c.b[1];
+        if (BEND) {
+            const double li = L * irho;
+            lam[0] = fma(-fma(li, irho, ay), lpx, fma(lirho, lam[5], lam[0]));
+            lam[4] = fma(li, lpx, lam[4]);
+        } else {
+            lam[0] = fma(-ay, lpx, lam[0]);
+        }
+        lam[2] = fma(ay, lpy, lam[2]);
+        if (c.sk >= 0) g = fma(L, fma(-x, lpx, y * lpy), g);     /* B_1, the only one */
+    } else {
+        adj_kick<BEND, AdjCoef<MO, false>>(c, x, y, L, lirho, irho, lam, g);
+    }
+}
+
 /* fastdrift (exact form) at input (px, py): x += nl px, y += nl py,
- * ct += nl S h with h = 1/(2 (1 + dp)); nl = L/(1 + dp_entry) is a function
- * of the element's entry momentum, collected in lnl */
-__device__ __forceinline__ void adj_fastdrift(double px, double py, double h, double nl,
-                                              double* lam, double& lnl) {
-    const double lx = lam[0], ly = lam[2], lc = lam[5];
-    const double S = fma(px, px, py * py);
-    const double c2 = 2.0 * lc * nl * h;
-    lam[1] += fma(lx, nl, c2 * px);
-    lam[3] += fma(ly, nl, c2 * py);
-    lam[4] -= c2 * S * h;
-    lnl += fma(lx, px, fma(ly, py, lc * S * h));
+ * ct += nl S h with h = 1/(2 (1 + dp)) and nl = L/(1 + dp_entry).  lam[5] is
+ * the same all through a magnet, so c2 = 2 h nl lam[5] comes from outside, and
+ * the momentum's share is left as two sums over the drifts of one length,
+ * a = sum lx px + ly py and b = sum S (adj_drift_sums). */
+struct DriftSums {
+    double a, b;
+};
+__device__ __forceinline__ void adj_fastdrift(double px, double py, double nl, double c2,
+                                              double* lam, DriftSums& d) {
+    const double lx = lam[0], ly = lam[2];
+    lam[1] = fma(lx, nl, fma(c2, px, lam[1]));
+    lam[3] = fma(ly, nl, fma(c2, py, lam[3]));
+    d.a = fma(lx, px, fma(ly, py, d.a));
+    d.b = fma(px, px, fma(py, py, d.b));
+}
+/* what drifts of length nl add to the cotangent of the body's momentum (from
+ * h), and to that of the entry's (from nl, times -1/(1 + dp_entry)) */
+__device__ __forceinline__ void adj_drift_sums(const DriftSums& d, double nl, double h, double lc,
+                                               double* lam, double& lnl) {
+    const double t = lc * h * d.b;
+    lam[4] = fma(-2.0 * nl * h, t, lam[4]);
+    lnl = fma(nl, d.a + t, lnl);
 }
 
 /* The transverse coordinates inside a non-radiating magnet, where dp is
- * constant and ct feeds nothing: what the recomputed steps carry. */
+ * constant and ct feeds nothing: what the undone stages carry.  They feed
+ * derivatives only and may differ from the tracked ones by roundings. */
 struct XY {
     double x, px, y, py;
 };
@@ -295,9 +350,9 @@ __device__ __forceinline__ void xy_drift(XY& q, double nl) {
     q.y = fma(nl, q.py, q.y);
 }
 
-template <bool BEND, int MO>
-__device__ __forceinline__ void xy_kick(XY& q, const AdjCoef<MO>& c, double L, double irho,
-                                        double dp) {
+/* a kick of length L; with -L, the kick undone */
+template <bool BEND, class C>
+__device__ __forceinline__ void xy_kick(XY& q, const C& c, double L, double irho, double dp) {
     double re, im;
     c.field(q.x, q.y, re, im);
     if (BEND) re = fma(-fma(-q.x, irho, dp), irho, re);     /* re - (dp - x irho) irho */
@@ -305,41 +360,41 @@ __device__ __forceinline__ void xy_kick(XY& q, const AdjCoef<MO>& c, double L, d
     q.py = fma(L, im, q.py);
 }
 
-/* one Forest-Ruth step (StrMPoleSymplectic4Pass.c:73-93) on the transverse
- * coordinates */
-template <bool BEND, int MO>
-__device__ __forceinline__ void xy_step(XY& q, const AdjCoef<MO>& c, double nl1, double nl2,
-                                        double K1, double K2, double irho, double dp) {
-    xy_drift(q, nl1);
-    xy_kick<BEND>(q, c, K1, irho, dp);
-    xy_drift(q, nl2);
-    xy_kick<BEND>(q, c, K2, irho, dp);
-    xy_drift(q, nl2);
-    xy_kick<BEND>(q, c, K1, irho, dp);
-    xy_drift(q, nl1);
-}
-
-/* edge_fringe (methods other than 3, exact arithmetic) at input s:
+/* edge_fringe (methods other than 3) at input (y, dp):
  * px += x fx, py -= y fy(dp) with fy = tn or tn/(1+dp) (method 2),
  * tn = irho tan(edge - fc/(1+dp)) (fy_c when that argument is the edge) */
-__device__ __forceinline__ void adj_edge(const P6& s, double* lam, double irho, double edge,
-                                         double fc, double fx, double fy_c, int method) {
-    const double opd = 1.0 + s.dp;
-    const double t = edge - fc / opd;
-    const double tn = (t == edge) ? fy_c : irho * tan(t);
-    double dtn = 0.0;
-    if (fc != 0.0) {
+__device__ __noinline__ double2 adj_edge_fringed(double dp, double irho, double edge, double fc,
+                                                 double fy_c, int method, bool fc0) {
+    const double opd = 1.0 + dp;
+    double fy = fy_c, dfy = 0.0;
+    if (!fc0) {
+        const double t = edge - fc / opd;
         const double tt = tan(t);
-        dtn = irho * fma(tt, tt, 1.0) * fc / (opd * opd);
+        if (t != edge) fy = irho * tt;
+        dfy = irho * fma(tt, tt, 1.0) * fc / (opd * opd);
     }
-    double fy = tn, dfy = dtn;
     if (method == ATB_BM_2) {
-        fy = tn / opd;
-        dfy = (dtn - fy) / opd;
+        fy = fy / opd;
+        dfy = (dfy - fy) / opd;
     }
-    lam[0] = fma(lam[1], fx, lam[0]);
-    lam[4] = fma(-lam[3] * s.y, dfy, lam[4]);
-    lam[2] = fma(-lam[3], fy, lam[2]);
+    return make_double2(fy, dfy);
+}
+__device__ __forceinline__ void adj_edge(double y, double dp, double* lam, double irho,
+                                         const Rec& e, int w_edge, int method, bool fc0) {
+    const double fy_c = e.f(w_edge + 3);
+    double2 f = make_double2(fy_c, 0.0);
+    if (!fc0 || method == ATB_BM_2)
+        f = adj_edge_fringed(dp, irho, e.f(w_edge), e.f(w_edge + 1), fy_c, method, fc0);
+    lam[0] = fma(lam[1], e.f(w_edge + 2), lam[0]);
+    lam[4] = fma(-lam[3] * y, f.y, lam[4]);
+    lam[2] = fma(-lam[3], f.x, lam[2]);
+}
+
+__device__ __forceinline__ double adj_edge_fy(double dp, double irho, const Rec& e, int w_edge,
+                                              int method, bool fc0) {
+    const double fy_c = e.f(w_edge + 3);
+    if (fc0 && method != ATB_BM_2) return fy_c;
+    return adj_edge_fringed(dp, irho, e.f(w_edge), e.f(w_edge + 1), fy_c, method, fc0).x;
 }
 
 /* the hand-written magnet path applies (flags and edge methods) */
@@ -355,105 +410,98 @@ __device__ __forceinline__ bool adj_by_hand(const Rec& e, bool bend) {
 }
 
 /* StrMPoleSymplectic4Pass.c:29-109 / BndMPoleSymplectic4Pass.c:38-129 in
- * reverse; `ss` is the thread's step-entry store.  The entry transforms run
- * in the tracking arithmetic from the stored entry state; the steps are
- * recomputed on the transverse coordinates. */
-template <bool BEND, int MO>
-__device__ __forceinline__ void adj_multipole_mo(const P6& s, double* lam, const Rec& e,
-                                                 const Param& pm, double& g,
-                                                 const StepStore& ss) {
+ * reverse, from the entry state s and the exit state sx.  A magnet with
+ * misalignments or apertures of its own finds the body's exit by tracking the
+ * body again (undoing a rotation would need its inverse). */
+template <bool BEND, int MO, bool SKEW>
+__device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Recip& rc,
+                                                 double* lam, const Rec& e, const Param& pm,
+                                                 double& g) {
     const uint32_t fl = e.flags();
-    const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2);
     const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
-    const int mo = e.mo();
+    const int mo = e.mo(), ns = e.nsteps();
     const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
-    AdjCoef<MO> c;
+    AdjCoef<MO, SKEW> c;
     c.load(A, A + mo + 1, mo, pm.k, pm.v);
+    const double pn0 = opd_rcp(rc, s.dp);
+    const double nl1 = e.f(ATB_SM_L1) * pn0, nl2 = e.f(ATB_SM_L2) * pn0, nl11 = 2.0 * nl1;
+    const double irho = BEND ? e.f(ATB_BM_IRHO) : 0.0;
+    const double k1i = BEND ? e.f(ATB_BM_K1IRHO) : 0.0, k2i = BEND ? e.f(ATB_BM_K2IRHO) : 0.0;
+    const int m_in = (int)((fl >> ATB_F_BM_IN_SHIFT) & ATB_F_BM_MASK);
+    const int m_out = (int)((fl >> ATB_F_BM_OUT_SHIFT) & ATB_F_BM_MASK);
 
-    /* forward to every step entry */
-    P6 r = s;
-    const double pn0 = 1.0 / (1.0 + r.dp);
-    const double nl1 = L1 * pn0, nl2 = L2 * pn0;
-    entrance_misalign(r, e);
-    const P6 s_in = r;                       /* entering the entrance edge */
-    double irho = 0.0, k1i = 0.0, k2i = 0.0;
-    int m_in = 0, m_out = 0;
-    if (BEND) {
-        irho = e.f(ATB_BM_IRHO);
-        k1i = e.f(ATB_BM_K1IRHO);
-        k2i = e.f(ATB_BM_K2IRHO);
-        m_in = (int)((fl >> ATB_F_BM_IN_SHIFT) & ATB_F_BM_MASK);
-        m_out = (int)((fl >> ATB_F_BM_OUT_SHIFT) & ATB_F_BM_MASK);
-        edge_fringe<false>(r, irho, e.f(ATB_BM_EIN), e.f(ATB_BM_FCIN), e.f(ATB_BM_FXIN),
-                           e.f(ATB_BM_FYIN), m_in, fl & ATB_F_FC0_IN, 1.0);
-    }
-    const double dp = r.dp;                  /* constant through the steps */
-    const double h = 1.0 / (2.0 * (1.0 + dp));
-    const int ns = e.nsteps();
-    const int stride = ns > ATB_ADJ_STEPS ? (ns + ATB_ADJ_STEPS - 1) / ATB_ADJ_STEPS : 1;
-    XY q{r.x, r.px, r.y, r.py};
-    for (int m = 0; m < ns; ++m) {
-        if (m % stride == 0) {
-            const int c = m / stride;
-            ss.at(c, 0) = q.x; ss.at(c, 1) = q.px; ss.at(c, 2) = q.y; ss.at(c, 3) = q.py;
+    /* q: leaving the body, before the exit edge */
+    XY q{sx.x, sx.px, sx.y, sx.py};
+    double dp = sx.dp;                       /* constant through the magnet */
+    if (e.opt) {
+        P6 r = s;
+        entrance_misalign(r, e);
+        dp = r.dp;
+        q = XY{r.x, r.px, r.y, r.py};
+        if (BEND) {
+            q.px = fma(q.x, e.f(ATB_BM_FXIN), q.px);
+            q.py = fma(-q.y, adj_edge_fy(dp, irho, e, ATB_BM_EIN, m_in, fl & ATB_F_FC0_IN), q.py);
         }
-        xy_step<BEND>(q, c, nl1, nl2, K1, K2, irho, dp);
+#pragma unroll 1
+        for (int i = 0; i < 3 * ns; ++i) {
+            const bool mid = i % 3 == 1;
+            xy_drift(q, i % 3 ? nl2 : i ? nl11 : nl1);
+            xy_kick<BEND>(q, c, mid ? K2 : K1, irho, dp);
+        }
+        if (ns > 0) xy_drift(q, nl1);
+        adj_exit_misalign(lam, e);
+    } else if (BEND) {
+        q.px = fma(-q.x, e.f(ATB_BM_FXOUT), q.px);
+        q.py = fma(q.y, adj_edge_fy(dp, irho, e, ATB_BM_EOUT, m_out, fl & ATB_F_FC0_OUT), q.py);
     }
-
-    /* reverse */
-    adj_exit_misalign(lam, e);
-    if (BEND) {
-        P6 so;
-        so.x = q.x; so.px = q.px; so.y = q.y; so.py = q.py; so.dp = dp; so.ct = 0.0;
-        adj_edge(so, lam, irho, e.f(ATB_BM_EOUT), e.f(ATB_BM_FCOUT), e.f(ATB_BM_FXOUT),
-                 e.f(ATB_BM_FYOUT), m_out);
+    const double h = 0.5 * (dp == s.dp ? pn0 : 1.0 / (1.0 + dp));
+    if (BEND) adj_edge(q.y, dp, lam, irho, e, ATB_BM_EOUT, m_out, fl & ATB_F_FC0_OUT);
+    double lnl = 0.0;
+    if (ns > 0) {
+        const double lc = lam[5], cc = 2.0 * h * lc;
+        const double c1 = cc * nl1, c2 = cc * nl2, c11 = cc * nl11;
+        DriftSums d1{0.0, 0.0}, d11{0.0, 0.0}, d2{0.0, 0.0};
+        adj_fastdrift(q.px, q.py, nl1, c1, lam, d1);
+        xy_drift(q, -nl1);
+        for (int m = ns;;) {
+            adj_kick<BEND>(c, q.x, q.y, K1, k1i, irho, lam, g);
+            xy_kick<BEND>(q, c, -K1, irho, dp);
+            adj_fastdrift(q.px, q.py, nl2, c2, lam, d2);
+            xy_drift(q, -nl2);
+            adj_kick<BEND>(c, q.x, q.y, K2, k2i, irho, lam, g);
+            xy_kick<BEND>(q, c, -K2, irho, dp);
+            adj_fastdrift(q.px, q.py, nl2, c2, lam, d2);
+            xy_drift(q, -nl2);
+            adj_kick<BEND>(c, q.x, q.y, K1, k1i, irho, lam, g);
+            xy_kick<BEND>(q, c, -K1, irho, dp);
+            if (--m == 0) break;
+            /* a step's first drift and the last of the step before it */
+            adj_fastdrift(q.px, q.py, nl11, c11, lam, d11);
+            xy_drift(q, -nl11);
+        }
+        adj_fastdrift(q.px, q.py, nl1, c1, lam, d1);
+        xy_drift(q, -nl1);
+        adj_drift_sums(d1, nl1, h, lc, lam, lnl);
+        adj_drift_sums(d11, nl11, h, lc, lam, lnl);
+        adj_drift_sums(d2, nl2, h, lc, lam, lnl);
     }
-    double lnl1 = 0.0, lnl2 = 0.0;
-    for (int m = ns - 1; m >= 0; --m) {
-        const int cb = m / stride;
-        XY t{ss.at(cb, 0), ss.at(cb, 1), ss.at(cb, 2), ss.at(cb, 3)};
-        for (int j = cb * stride; j < m; ++j) xy_step<BEND>(t, c, nl1, nl2, K1, K2, irho, dp);
-        /* the step once more, keeping the input of every stage */
-        const double px0 = t.px, py0 = t.py;
-        xy_drift(t, nl1);
-        const double x1 = t.x, y1 = t.y;
-        xy_kick<BEND>(t, c, K1, irho, dp);
-        const double px2 = t.px, py2 = t.py;
-        xy_drift(t, nl2);
-        const double x3 = t.x, y3 = t.y;
-        xy_kick<BEND>(t, c, K2, irho, dp);
-        const double px4 = t.px, py4 = t.py;
-        xy_drift(t, nl2);
-        const double x5 = t.x, y5 = t.y;
-        xy_kick<BEND>(t, c, K1, irho, dp);
-        const double px6 = t.px, py6 = t.py;
-        adj_fastdrift(px6, py6, h, nl1, lam, lnl1);
-        adj_kick<BEND>(c, x5, y5, K1, k1i, irho, lam, g);
-        adj_fastdrift(px4, py4, h, nl2, lam, lnl2);
-        adj_kick<BEND>(c, x3, y3, K2, k2i, irho, lam, g);
-        adj_fastdrift(px2, py2, h, nl2, lam, lnl2);
-        adj_kick<BEND>(c, x1, y1, K1, k1i, irho, lam, g);
-        adj_fastdrift(px0, py0, h, nl1, lam, lnl1);
-    }
-    if (BEND)
-        adj_edge(s_in, lam, irho, e.f(ATB_BM_EIN), e.f(ATB_BM_FCIN), e.f(ATB_BM_FXIN),
-                 e.f(ATB_BM_FYIN), m_in);
-    adj_entrance_misalign(lam, e);
-    /* nl1, nl2 = L1, L2 / (1 + dp) of the entry momentum */
-    lam[4] -= fma(lnl1, L1, lnl2 * L2) * pn0 * pn0;
+    if (BEND) adj_edge(q.y, dp, lam, irho, e, ATB_BM_EIN, m_in, fl & ATB_F_FC0_IN);
+    if (e.opt) adj_entrance_misalign(lam, e);
+    /* nl = L / (1 + dp) of the entry momentum */
+    lam[4] = fma(-lnl, pn0, lam[4]);
 }
 
 template <bool BEND>
-__device__ __forceinline__ void adj_pass_multipole(const P6& s, double* lam, const Rec& e,
-                                                   const Param& pm, double& g,
-                                                   const StepStore& ss) {
-    switch (e.mo()) {
-        case 0: adj_multipole_mo<BEND, 0>(s, lam, e, pm, g, ss); break;
-        case 1: adj_multipole_mo<BEND, 1>(s, lam, e, pm, g, ss); break;
-        case 2: adj_multipole_mo<BEND, 2>(s, lam, e, pm, g, ss); break;
-        case 3: adj_multipole_mo<BEND, 3>(s, lam, e, pm, g, ss); break;
-        default: adj_multipole_mo<BEND, -1>(s, lam, e, pm, g, ss); break;
-    }
+__device__ __forceinline__ void adj_pass_multipole(const P6& s, const P6& sx, Recip& rc,
+                                                   double* lam, const Rec& e, const Param& pm,
+                                                   double& g) {
+    const bool upright = e.flags() & ATB_F_NOSKEW;
+    const int mo = e.mo();
+    if (mo == 1 && upright) adj_multipole_mo<BEND, 1, false>(s, sx, rc, lam, e, pm, g);
+    else if (mo == 2 && upright) adj_multipole_mo<BEND, 2, false>(s, sx, rc, lam, e, pm, g);
+    else if (mo == 3 && upright) adj_multipole_mo<BEND, 3, false>(s, sx, rc, lam, e, pm, g);
+    else if (mo == 0) adj_multipole_mo<BEND, 0, true>(s, sx, rc, lam, e, pm, g);
+    else adj_multipole_mo<BEND, -1, true>(s, sx, rc, lam, e, pm, g);
 }
 
 /* ---- thin elements -------------------------------------------------------- */
@@ -479,9 +527,9 @@ __device__ __forceinline__ void adj_pass_rfcavity(const P6& s, double* lam, cons
     drift6<false>(r, half);
     const P6 s1 = r;
     if (fl & ATB_F_NV) rf_kick(r, e, nturn);
-    adj_drift6(r, lam, half);
+    adj_drift6(r, lam, half, 1.0 / (1.0 + r.dp));
     if (fl & ATB_F_NV) adj_rf_kick(s1, lam, e, nturn);
-    adj_drift6(s, lam, half);
+    adj_drift6(s, lam, half, 1.0 / (1.0 + s.dp));
 }
 
 /* ThinMPolePass.c:28-70 without field scaling */
@@ -498,7 +546,7 @@ __device__ __forceinline__ void adj_pass_thinmpole(const P6& s, double* lam, con
     lam[4] = fma(bax, lam[1], fma(-bay, lam[3], lam[4]));
     lam[0] = fma(-bax, lam[5], lam[0]);
     lam[2] = fma(bay, lam[5], lam[2]);
-    AdjCoef<-1> c;
+    AdjCoef<-1, true> c;
     c.load(A, B, mo, pm.k, pm.v);
     adj_kick<false>(c, r.x, r.y, 1.0, 0.0, 0.0, lam, g);
     adj_entrance_misalign(lam, e);
@@ -542,11 +590,12 @@ __device__ __noinline__ Lam6 adj_dual7(P6 s, Lam6 in, Rec e, int nturn, Param pm
     return adj_dual<7>(s, in, e, nturn, pm);
 }
 
-/* lambda <- J_e(s)^T lambda; g += the strength's term */
-__device__ __forceinline__ void adj_element(const P6& s, double* lam, const Rec& e, int nturn,
-                                            const Param& pm, double& g, const StepStore& ss) {
+/* lambda <- J_e(s)^T lambda; g += the strength's term; sx: the exit state */
+__device__ __forceinline__ void adj_element(const P6& s, const P6& sx, Recip& rc, double* lam,
+                                            const Rec& e, int nturn, const Param& pm,
+                                            double& g) {
     switch (e.op()) {
-        case ATB_OP_DRIFT: adj_pass_drift(s, lam, e); return;
+        case ATB_OP_DRIFT: adj_pass_drift(s, rc, lam, e); return;
         case ATB_OP_IDENTITY:
             adj_exit_misalign(lam, e);
             adj_entrance_misalign(lam, e);
@@ -565,10 +614,10 @@ __device__ __forceinline__ void adj_element(const P6& s, double* lam, const Rec&
             if (!(e.flags() & ATB_F_SCALING)) { adj_pass_thinmpole(s, lam, e, pm, g); return; }
             break;
         case ATB_OP_STRMPOLE:
-            if (adj_by_hand(e, false)) { adj_pass_multipole<false>(s, lam, e, pm, g, ss); return; }
+            if (adj_by_hand(e, false)) { adj_pass_multipole<false>(s, sx, rc, lam, e, pm, g); return; }
             break;
         case ATB_OP_BNDMPOLE:
-            if (adj_by_hand(e, true)) { adj_pass_multipole<true>(s, lam, e, pm, g, ss); return; }
+            if (adj_by_hand(e, true)) { adj_pass_multipole<true>(s, sx, rc, lam, e, pm, g); return; }
             break;
         default: break;
     }
@@ -622,48 +671,39 @@ atb_adjoint_forward_kernel(const AtbAdjoint A) {
 
 extern "C" __global__ void __launch_bounds__(ATB_ADJ_THREADS, ATB_ADJ_MIN_BLOCKS)
 atb_adjoint_turn_kernel(const AtbAdjoint A) {
-    /* the block's strength gradient (nparam words), then the threads' step
-       stores (ATB_ADJ_STEPS x 4 x blockDim words) */
+    /* the block's strength gradient (nparam words) */
     extern __shared__ double sg[];
     for (int q = threadIdx.x; q < A.nparam; q += blockDim.x) sg[q] = 0.0;
     __syncthreads();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = p < A.np;
     const long long np = A.np;
-    P6 s;
+    P6 exit;                      /* leaving the element at hand */
     double lam[6];
     bool live = false;
     if (in) {
-        load6(A.ckpt + 6 * p, s);
+        /* a particle lost during the turn enters the next one as NaN */
+        live = !isnan(__ldg(A.ckpt + 6 * p));
+        load6(A.next + 6 * p, exit);
+        live &= !isnan(exit.x);
 #pragma unroll
         for (int i = 0; i < 6; ++i) lam[i] = A.lam[6 * p + i];
-        live = !isnan(s.x);
 #pragma unroll
         for (int i = 0; i < 6; ++i) live &= isfinite(lam[i]);
     }
-    if (A.next) {
-        /* the forward pass stored this turn's element-entry states; a
-           particle lost during the turn enters the next one as NaN */
-        if (live) live = !isnan(__ldg(A.next + 6 * p));
-    } else {
-        /* the turn once more, every element's entry state to the scratch */
-        Recip rc;
-        for (int ei = 0; ei < A.nelem; ++ei) {
-            if (live) {
-                store6(A.scratch + 6 * ((long long)ei * np + p), s);
-                track_element(s, rc, adj_rec(A, ei), A.turn0, adj_param(A, ei));
-                if (is_bad(s)) live = false;      /* lost in this turn */
-            }
-        }
-    }
-    const StepStore ss{sg + A.nparam + threadIdx.x, (int)blockDim.x};
+    /* an element's entry state is asked for while the one behind it is worked
+       on: it comes from HBM */
+    P6 ahead;
+    Recip rc;
+    if (live && A.nelem > 0) load6(A.scratch + 6 * ((long long)(A.nelem - 1) * np + p), ahead);
     for (int ei = A.nelem - 1; ei >= 0; --ei) {
         const Param pm = adj_param(A, ei);
         double g = 0.0;
         if (live) {
-            P6 se;
-            load6(A.scratch + 6 * ((long long)ei * np + p), se);
-            adj_element(se, lam, adj_rec(A, ei), A.turn0, pm, g, ss);
+            const P6 se = ahead;
+            if (ei > 0) load6(A.scratch + 6 * ((long long)(ei - 1) * np + p), ahead);
+            adj_element(se, exit, rc, lam, adj_rec(A, ei), A.turn0, pm, g);
+            exit = se;
         }
         if (pm.k >= 0) {                      /* the same for the whole block */
             g = warp_sum(g);

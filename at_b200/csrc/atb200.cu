@@ -157,7 +157,7 @@ struct atb_handle {
     std::vector<Lattice> lats;
     DevBuf r, rout, lost, lturn, lelem, lcoord, refpts, jobs, tiles, counter, status, alive,
         moments, tan_pelem, tan_porder, compact, jobnext, adj_pelem, adj_porder, adj_scratch,
-        adj_block, adj_state;
+        adj_block, adj_state, adj_next;
     std::vector<int32_t> h_pelem;
     std::vector<AtbTile> h_tiles;
     std::vector<struct Batch> batches;
@@ -585,7 +585,7 @@ int atb_destroy(atb_handle* h) {
                           &h->refpts, &h->jobs, &h->tiles, &h->counter, &h->status, &h->alive,
                           &h->moments, &h->tan_pelem, &h->tan_porder, &h->compact,
                           &h->adj_pelem, &h->adj_porder, &h->adj_scratch, &h->adj_block,
-                          &h->adj_state,
+                          &h->adj_state, &h->adj_next,
                           &h->jobnext})
             b->release();
         for (int i = 0; i < 2; ++i) {
@@ -1241,8 +1241,7 @@ int atb_adjoint_backward(atb_handle* h, int32_t id, const double* ckpt, int64_t 
     if (estates && (stride != 1 || !rfinal))
         return fail(ATB_ERR_ARG, "element states need a checkpoint every turn and the final "
                                  "states");
-    if (((size_t)nparam + (size_t)ATB_ADJ_STEPS_SMEM * 4 * ATB_ADJ_THREADS) * sizeof(double) >
-        48 * 1024)
+    if (nparam > ATB_ADJ_MAX_PARAMS)
         return fail(ATB_ERR_ARG, "at most 1024 strengths");
     if (np > (int64_t)ATB_ADJ_THREADS * 0x7fffffffLL) return fail(ATB_ERR_ARG, "too many particles");
     const int rc = strength_map(h, L, param_elem, param_order, nparam, "adjoint");
@@ -1254,8 +1253,7 @@ int atb_adjoint_backward(atb_handle* h, int32_t id, const double* ckpt, int64_t 
     AtbAdjoint A;
     const int rs = adjoint_setup(h, L, param_order, param_value, nparam, st, A);
     if (rs != ATB_OK) return rs;
-    const size_t smem_e =
-        ((size_t)nparam + (size_t)ATB_ADJ_STEPS_SMEM * 4 * ATB_ADJ_THREADS) * sizeof(double);
+    const size_t smem = (size_t)nparam * sizeof(double);
     if (estates) {
         /* every turn's element-entry states were stored by the forward pass:
            no tracking here, all particles in one launch per turn */
@@ -1268,7 +1266,7 @@ int atb_adjoint_backward(atb_handle* h, int32_t id, const double* ckpt, int64_t 
             T.turn0 = turn0 + t;
             T.scratch = const_cast<double*>(estates) + 6 * ((int64_t)t * L->nelem * np);
             T.next = (t + 1 < nturns) ? ckpt + 6 * ((int64_t)(t + 1) * np) : rfinal;
-            atb_adjoint_turn_kernel<<<adjoint_blocks(np), ATB_ADJ_THREADS, smem_e, st>>>(T);
+            atb_adjoint_turn_kernel<<<adjoint_blocks(np), ATB_ADJ_THREADS, smem, st>>>(T);
         }
         ATB_CUDA(cudaGetLastError());
         return ATB_OK;
@@ -1276,17 +1274,43 @@ int atb_adjoint_backward(atb_handle* h, int32_t id, const double* ckpt, int64_t 
     /* particles in chunks whose element-entry scratch fits 8 GiB */
     const int64_t per = (int64_t)std::max(L->nelem, 1) * 6 * sizeof(double);
     const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(np, (8LL << 30) / per));
-    if (h->adj_scratch.ensure((size_t)(chunk * per)) != cudaSuccess)
+    if (h->adj_scratch.ensure((size_t)(chunk * per)) != cudaSuccess ||
+        h->adj_next.ensure((size_t)chunk * 6 * sizeof(double)) != cudaSuccess)
         return fail(ATB_ERR_NOMEM, "cudaMalloc(adjoint scratch) failed");
     if (stride > 1 &&
         (h->adj_block.ensure((size_t)stride * chunk * 6 * sizeof(double)) != cudaSuccess ||
          h->adj_state.ensure((size_t)chunk * 6 * sizeof(double)) != cudaSuccess))
         return fail(ATB_ERR_NOMEM, "cudaMalloc(adjoint checkpoints) failed");
     const int nck = (nturns + stride - 1) / stride;
-    const size_t smem =
-        ((size_t)nparam + (size_t)ATB_ADJ_STEPS_SMEM * 4 * ATB_ADJ_THREADS) * sizeof(double);
     A.gparam = gparam;
     A.scratch = h->adj_scratch.as<double>();
+    /* One turn backwards from its entry states: tracked again by the forward
+       kernel, which stores the element-entry states, then swept.  (In one
+       kernel the two shared 128 registers and an instruction cache that holds
+       neither: with the same sweep 3.6 ms for 65,536 particles and a turn of
+       the FODO ring, in two launches 3.1 ms.) */
+    auto turn_back = [&](double* entry, int64_t n, double* lp, int turn) -> cudaError_t {
+        double* next = h->adj_next.as<double>();
+        cudaError_t e = cudaMemcpyAsync(next, entry, (size_t)n * 6 * sizeof(double),
+                                        cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) return e;
+        AtbAdjoint F = A;
+        F.np = n;
+        F.ld = n;
+        F.r = next;
+        F.nturns = 1;
+        F.turn0 = turn;
+        F.stride = 1;
+        atb_adjoint_forward_kernel<<<adjoint_blocks(n), ATB_ADJ_THREADS, 0, st>>>(F);
+        AtbAdjoint T = A;
+        T.np = n;
+        T.ckpt = entry;
+        T.next = next;
+        T.lam = lp;
+        T.turn0 = turn;
+        atb_adjoint_turn_kernel<<<adjoint_blocks(n), ATB_ADJ_THREADS, smem, st>>>(T);
+        return cudaSuccess;
+    };
     for (int64_t p0 = 0; p0 < np; p0 += chunk) {
         const int64_t n = std::min(chunk, np - p0);
         double* lp = lam + 6 * p0;
@@ -1295,12 +1319,7 @@ int atb_adjoint_backward(atb_handle* h, int32_t id, const double* ckpt, int64_t 
             const int nt = std::min(stride, nturns - t0);
             const double* slab = ckpt + 6 * ((int64_t)b * np + p0);
             if (stride == 1) {
-                AtbAdjoint T = A;
-                T.np = n;
-                T.ckpt = const_cast<double*>(slab);
-                T.lam = lp;
-                T.turn0 = turn0 + t0;
-                atb_adjoint_turn_kernel<<<adjoint_blocks(n), ATB_ADJ_THREADS, smem, st>>>(T);
+                ATB_CUDA(turn_back(const_cast<double*>(slab), n, lp, turn0 + t0));
                 continue;
             }
             /* the block's turn entries, tracked again from its checkpoint */
@@ -1319,14 +1338,8 @@ int atb_adjoint_backward(atb_handle* h, int32_t id, const double* ckpt, int64_t 
             F.skip_last = 1;
             F.scratch = nullptr;       /* no element states from this re-tracking */
             atb_adjoint_forward_kernel<<<adjoint_blocks(n), ATB_ADJ_THREADS, 0, st>>>(F);
-            for (int t = nt - 1; t >= 0; --t) {
-                AtbAdjoint T = A;
-                T.np = n;
-                T.ckpt = blk + 6 * ((int64_t)t * n);
-                T.lam = lp;
-                T.turn0 = turn0 + t0 + t;
-                atb_adjoint_turn_kernel<<<adjoint_blocks(n), ATB_ADJ_THREADS, smem, st>>>(T);
-            }
+            for (int t = nt - 1; t >= 0; --t)
+                ATB_CUDA(turn_back(blk + 6 * ((int64_t)t * n), n, lp, turn0 + t0 + t));
         }
     }
     ATB_CUDA(cudaGetLastError());

@@ -175,13 +175,12 @@ typedef struct AtbTangent {
  * kernel tracks `nturns` turns with the differentiated strengths substituted
  * and stores the state entering every `stride`-th turn in `ckpt`
  * ((turns / stride, ld, 6) slabs).  The turn kernel runs the adjoint of one
- * turn (absolute number turn0) from its entry states `ckpt` ((np, 6)): it
- * re-tracks the turn storing every element's entry state in `scratch`
- * ((nelem, np, 6)), then maps the cotangent `lam` ((np, 6), in place) from
- * the turn's exit to its entry and adds the strengths' gradient to
- * `gparam`. */
+ * turn (absolute number turn0) from its entry states `ckpt` ((np, 6)) and
+ * every element's entry states `scratch` ((nelem, np, 6)), which the forward
+ * kernel stored: it maps the cotangent `lam` ((np, 6), in place) from the
+ * turn's exit to its entry and adds the strengths' gradient to `gparam`. */
 #define ATB_ADJ_THREADS 128
-#define ATB_ADJ_STEPS_SMEM 10      /* step entries a thread keeps in shared memory */
+#define ATB_ADJ_MAX_PARAMS 1024    /* strengths whose sums a block keeps */
 
 typedef struct AtbAdjoint {
     const double* table;        /* element table words                      */
@@ -207,10 +206,8 @@ typedef struct AtbAdjoint {
                                    ((nturns, nelem, ld, 6)), stored as the
                                    particles pass                          */
     double* gparam;             /* turn kernel: (nparam), added to          */
-    const double* next;         /* turn kernel, states stored by the forward
-                                   pass: the (np, 6) states entering the next
-                                   turn (NaN: lost in this one); NULL: the
-                                   kernel tracks the turn again itself      */
+    const double* next;         /* turn kernel: the (np, 6) states entering
+                                   the next turn (NaN: lost in this one)   */
 } AtbAdjoint;
 
 /* Per-element transfer and diffusion matrices for a particle entering each
