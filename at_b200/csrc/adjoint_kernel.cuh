@@ -413,7 +413,7 @@ __device__ __forceinline__ bool adj_by_hand(const Rec& e, bool bend) {
  * reverse, from the entry state s and the exit state sx.  A magnet with
  * misalignments or apertures of its own finds the body's exit by tracking the
  * body again (undoing a rotation would need its inverse). */
-template <bool BEND, int MO, bool SKEW>
+template <bool BEND, int MO, bool SKEW, bool PLAIN = false>
 __device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Recip& rc,
                                                  double* lam, const Rec& e, const Param& pm,
                                                  double& g) {
@@ -433,7 +433,7 @@ __device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Reci
     /* q: leaving the body, before the exit edge */
     XY q{sx.x, sx.px, sx.y, sx.py};
     double dp = sx.dp;                       /* constant through the magnet */
-    if (e.opt) {
+    if (!PLAIN && e.opt) {
         P6 r = s;
         entrance_misalign(r, e);
         dp = r.dp;
@@ -454,7 +454,7 @@ __device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Reci
         q.px = fma(-q.x, e.f(ATB_BM_FXOUT), q.px);
         q.py = fma(q.y, adj_edge_fy(dp, irho, e, ATB_BM_EOUT, m_out, fl & ATB_F_FC0_OUT), q.py);
     }
-    const double h = 0.5 * (dp == s.dp ? pn0 : 1.0 / (1.0 + dp));
+    const double h = 0.5 * (PLAIN || dp == s.dp ? pn0 : 1.0 / (1.0 + dp));
     if (BEND) adj_edge(q.y, dp, lam, irho, e, ATB_BM_EOUT, m_out, fl & ATB_F_FC0_OUT);
     double lnl = 0.0;
     if (ns > 0) {
@@ -486,7 +486,7 @@ __device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Reci
         adj_drift_sums(d2, nl2, h, lc, lam, lnl);
     }
     if (BEND) adj_edge(q.y, dp, lam, irho, e, ATB_BM_EIN, m_in, fl & ATB_F_FC0_IN);
-    if (e.opt) adj_entrance_misalign(lam, e);
+    if (!PLAIN && e.opt) adj_entrance_misalign(lam, e);
     /* nl = L / (1 + dp) of the entry momentum */
     lam[4] = fma(-lnl, pn0, lam[4]);
 }
@@ -590,10 +590,8 @@ __device__ __noinline__ Lam6 adj_dual7(P6 s, Lam6 in, Rec e, int nturn, Param pm
     return adj_dual<7>(s, in, e, nturn, pm);
 }
 
-/* lambda <- J_e(s)^T lambda; g += the strength's term; sx: the exit state */
-__device__ __forceinline__ void adj_element(const P6& s, const P6& sx, Recip& rc, double* lam,
-                                            const Rec& e, int nturn, const Param& pm,
-                                            double& g) {
+__device__ __forceinline__ void adj_any(const P6& s, const P6& sx, Recip& rc, double* lam,
+                                        const Rec& e, int nturn, const Param& pm, double& g) {
     switch (e.op()) {
         case ATB_OP_DRIFT: adj_pass_drift(s, rc, lam, e); return;
         case ATB_OP_IDENTITY:
@@ -629,6 +627,45 @@ __device__ __forceinline__ void adj_element(const P6& s, const P6& sx, Recip& rc
 #pragma unroll
     for (int i = 0; i < 6; ++i) lam[i] = out.v[i];
     g += out.g;
+}
+
+/* any element, out of line: what most of a ring's elements do not need would
+ * otherwise have the sweep's state spilled around every one of them */
+__device__ __noinline__ Lam6 adj_rare(P6 s, P6 sx, double pn, Lam6 in, Rec e, int nturn,
+                                      Param pm) {
+    Recip rc;
+    rc.dp = s.dp;
+    rc.pn = pn;
+    adj_any(s, sx, rc, in.v, e, nturn, pm, in.g);
+    return in;
+}
+
+/* lambda <- J_e(s)^T lambda; g += the strength's term; sx: the exit state */
+__device__ __forceinline__ void adj_element(const P6& s, const P6& sx, Recip& rc, double* lam,
+                                            const Rec& e, int nturn, const Param& pm,
+                                            double& g) {
+    const int op = e.op(), mo = e.mo();
+    const bool plain = e.opt == 0, upright = e.flags() & ATB_F_NOSKEW;
+    if (op == ATB_OP_DRIFT && plain) {
+        adj_drift6(s, lam, e.f(ATB_DR_LE), opd_rcp(rc, s.dp));
+        return;
+    }
+    if (op == ATB_OP_STRMPOLE && plain && upright && adj_by_hand(e, false)) {
+        if (mo == 1) { adj_multipole_mo<false, 1, false, true>(s, sx, rc, lam, e, pm, g); return; }
+        if (mo == 2) { adj_multipole_mo<false, 2, false, true>(s, sx, rc, lam, e, pm, g); return; }
+    }
+    if (op == ATB_OP_BNDMPOLE && plain && upright && mo == 1 && adj_by_hand(e, true)) {
+        adj_multipole_mo<true, 1, false, true>(s, sx, rc, lam, e, pm, g);
+        return;
+    }
+    Lam6 io;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) io.v[i] = lam[i];
+    io.g = g;
+    io = adj_rare(s, sx, opd_rcp(rc, s.dp), io, e, nturn, pm);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) lam[i] = io.v[i];
+    g = io.g;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
