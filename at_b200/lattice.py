@@ -57,14 +57,13 @@ LIMIT_AMPLITUDE = 1.0
 _f64 = np.float64
 
 
-def _ieee(op, a, b):
-    """One IEEE double operation with C semantics (no Python exceptions)."""
-    with np.errstate(all="ignore"):
-        return float(op(_f64(a), _f64(b)))
-
-
 def _div(a, b):
-    return _ieee(np.divide, a, b)
+    """One IEEE double division with C semantics (no Python exceptions)."""
+    try:
+        return float(a) / float(b)
+    except ZeroDivisionError:
+        with np.errstate(all="ignore"):
+            return float(np.divide(_f64(a), _f64(b)))
 
 
 def c_round(x: float) -> float:
@@ -88,17 +87,22 @@ def _get_long(el, name: str) -> int:
     return operator.index(getattr(el, name))            # atelem.c:219-226
 
 
+_MISSING = object()      # an absent attribute costs no exception
+
+
 def _opt_double(el, name: str, default: float) -> float:
     try:
-        return _get_double(el, name)
-    except (AttributeError, TypeError, ValueError):     # atelem.c:247-255
+        v = getattr(el, name, _MISSING)                 # atelem.c:247-255
+        return default if v is _MISSING else float(v)
+    except (AttributeError, TypeError, ValueError):
         return default
 
 
 def _opt_long(el, name: str, default: int) -> int:
     try:
-        return _get_long(el, name)
-    except (AttributeError, TypeError, ValueError):     # atelem.c:237-245
+        v = getattr(el, name, _MISSING)                 # atelem.c:237-245
+        return default if v is _MISSING else operator.index(v)
+    except (AttributeError, TypeError, ValueError):
         return default
 
 
@@ -108,7 +112,8 @@ def _check_array(a, name: str) -> np.ndarray:
         raise RuntimeError("The attribute %s is not an array." % name)
     if a.dtype != np.float64:
         raise RuntimeError("The attribute %s is not a double array." % name)
-    if not (a.flags.f_contiguous and a.flags.aligned):
+    flags = a.flags
+    if not (flags.f_contiguous and flags.aligned):
         raise RuntimeError("The attribute %s is not Fortran-aligned." % name)
     return a.ravel(order="F")
 
@@ -118,9 +123,8 @@ def _get_array(el, name: str) -> np.ndarray:
 
 
 def _opt_array(el, name: str):
-    try:
-        a = getattr(el, name)                           # atelem.c:336-346
-    except AttributeError:
+    a = getattr(el, name, _MISSING)                     # atelem.c:336-346
+    if a is _MISSING:
         return None
     return _check_array(a, name)
 
@@ -142,20 +146,19 @@ def _pack_header(op: int, max_order: int, flags: int, nsteps: int, nwords: int) 
             | (nwords & T.ATB_H_LEN_MASK) << T.ATB_H_LEN_SHIFT)
 
 
-def _tilt_pattern(r: np.ndarray):
+# places of a column-major 6x6: what a rotation of the x/y planes holds, and
+# the entries that must be zero beside the ones at [4, 4] and [5, 5]
+_TILT = ((0, 0), (0, 2), (1, 1), (1, 3), (2, 0), (2, 2), (3, 1), (3, 3))
+_tilt_kept = operator.itemgetter(*(i + 6 * j for i, j in _TILT))
+_tilt_zero = operator.itemgetter(*(i + 6 * j for j in range(6) for i in range(6)
+                                   if (i, j) not in _TILT and not (i == j and i >= 4)))
+
+
+def _tilt_pattern(r: list):
     """8 rotation entries if the 6x6 (column-major) R only couples x/y planes."""
-    m = r.reshape(6, 6, order="F")
-    keep = {(0, 0), (0, 2), (1, 1), (1, 3), (2, 0), (2, 2), (3, 1), (3, 3)}
-    for i in range(6):
-        for j in range(6):
-            if (i, j) in keep:
-                continue
-            if i == j and i >= 4:
-                if m[i, j] != 1.0:
-                    return None
-            elif m[i, j] != 0.0:
-                return None
-    return [m[0, 0], m[0, 2], m[1, 1], m[1, 3], m[2, 0], m[2, 2], m[3, 1], m[3, 3]]
+    if r[28] != 1.0 or r[35] != 1.0 or any(_tilt_zero(r)):
+        return None
+    return _tilt_kept(r)
 
 
 class _Record:
@@ -168,38 +171,42 @@ class _Record:
         self.blocks: list[tuple[int, list[float]]] = []
 
     def set(self, word: int, value: float):
-        while len(self.fields) <= word:
-            self.fields.append(0.0)
         self.fields[word] = float(value)
 
-    def add_block(self, slot: int, values):
-        self.blocks.append((slot, [float(v) for v in values]))
+    def reserve(self, nwords: int):
+        self.fields.extend([0.0] * (nwords - len(self.fields)))
 
-    def words(self) -> np.ndarray:
-        body = list(self.fields[2:])
-        pos = 2 + len(body)
-        offs = [0] * T.ATB_NUM_OPT
+    def add_block(self, slot: int, values):
+        self.blocks.append((slot, values))
+
+    def emit(self, out: list) -> tuple[int, int, int]:
+        """Append the record to ``out`` (zeros in the place of the two header
+        words); returns the header words and the record's length."""
+        fields = self.fields
+        pos = len(fields)
+        out.extend(fields)
+        optw = 0
         for slot, vals in self.blocks:
             if pos % 2:                      # 16-byte align every block
-                body.append(0.0)
+                out.append(0.0)
                 pos += 1
-            offs[slot] = pos
-            body.extend(vals)
+            optw |= (pos & T.ATB_OPT_MASK) << (slot * T.ATB_OPT_BITS)
+            out.extend(vals)
             pos += len(vals)
         if pos % 2:
-            body.append(0.0)
+            out.append(0.0)
             pos += 1
-        if pos > T.ATB_MAX_RECORD_WORDS:
-            raise ValueError("element record too long (%d words)" % pos)
-        out = np.zeros(pos, dtype=np.float64)
-        out[2:] = body
-        u = out.view(np.uint64)
-        u[0] = _pack_header(self.op, self.max_order, self.flags, self.nsteps, pos)
-        optw = 0
-        for s, o in enumerate(offs):
-            optw |= (o & T.ATB_OPT_MASK) << (s * T.ATB_OPT_BITS)
-        u[1] = optw
-        return out
+        return _pack_header(self.op, self.max_order, self.flags, self.nsteps, pos), optw, pos
+
+
+def _add_rotation(rec: _Record, r, slot: int, dense: int):
+    r = r[:36].tolist()
+    tilt = _tilt_pattern(r)
+    if tilt is None:
+        rec.flags |= dense
+        rec.add_block(slot, r)
+    else:
+        rec.add_block(slot, tilt)
 
 
 def _add_misalign_entrance(rec: _Record, el):
@@ -210,27 +217,17 @@ def _add_misalign_entrance(rec: _Record, el):
     r2 = _need(_opt_array(el, "R2"), 36, "R2")
     t2 = _need(_opt_array(el, "T2"), 6, "T2")
     if t1 is not None:
-        rec.add_block(T.ATB_OPT_T1, t1[:6])
+        rec.add_block(T.ATB_OPT_T1, t1[:6].tolist())
     if r1 is not None:
-        tilt = _tilt_pattern(r1[:36])
-        if tilt is None:
-            rec.flags |= T.ATB_F_R1_DENSE
-            rec.add_block(T.ATB_OPT_R1, r1[:36])
-        else:
-            rec.add_block(T.ATB_OPT_R1, tilt)
+        _add_rotation(rec, r1, T.ATB_OPT_R1, T.ATB_F_R1_DENSE)
     if rap is not None:
-        rec.add_block(T.ATB_OPT_RAP, rap[:4])
+        rec.add_block(T.ATB_OPT_RAP, rap[:4].tolist())
     if eap is not None:
-        rec.add_block(T.ATB_OPT_EAP, eap[:2])
+        rec.add_block(T.ATB_OPT_EAP, eap[:2].tolist())
     if r2 is not None:
-        tilt = _tilt_pattern(r2[:36])
-        if tilt is None:
-            rec.flags |= T.ATB_F_R2_DENSE
-            rec.add_block(T.ATB_OPT_R2, r2[:36])
-        else:
-            rec.add_block(T.ATB_OPT_R2, tilt)
+        _add_rotation(rec, r2, T.ATB_OPT_R2, T.ATB_F_R2_DENSE)
     if t2 is not None:
-        rec.add_block(T.ATB_OPT_T2, t2[:6])
+        rec.add_block(T.ATB_OPT_T2, t2[:6].tolist())
 
 
 def _fringe_matrix(k1: float, fint: np.ndarray, part: int):
@@ -314,8 +311,8 @@ def _multipole_common(rec: _Record, el, op: int, bend: bool, integrator: int = 4
         raise ValueError("NumIntSteps %d out of range" % ns)
     _need(pa, mo + 1, "PolynomA")
     _need(pb, mo + 1, "PolynomB")
-    A = [float(v) for v in pa[: mo + 1]]
-    B = [float(v) for v in pb[: mo + 1]]
+    A = pa[: mo + 1].tolist()
+    B = pb[: mo + 1].tolist()
     b1_fringe = float(pb[1]) if pb.size > 1 else 0.0
     # StrMPoleSymplectic4Pass.c:39-52 (same lines in the Bnd and Rad variants)
     sl = _div(le, ns)
@@ -389,11 +386,9 @@ def _multipole_common(rec: _Record, el, op: int, bend: bool, integrator: int = 4
         base = T.ATB_BM_POLY
     else:
         base = T.ATB_SM_POLY
-    for i, v in enumerate(A):
-        rec.set(base + i, v)
-    for i, v in enumerate(B):
-        rec.set(base + mo + 1 + i, v)
-    if all(v == 0.0 for v in A):
+    rec.reserve(base)
+    rec.fields[base:] = A + B
+    if not any(A):
         rec.flags |= T.ATB_F_NOSKEW
 
 
@@ -422,6 +417,8 @@ class CompiledLattice:
     #: (word index, element index, kind) of energy-dependent fields
     energy_fields: list[tuple[int, int, str]] = field(default_factory=list)
     voltages: dict[int, float] = field(default_factory=dict)
+    #: no element holds an error (False: not known)
+    clean: bool = False
 
     @property
     def nelem(self) -> int:
@@ -429,7 +426,7 @@ class CompiledLattice:
 
     def first_error(self, start: int, end: int, nturns: int):
         """The error the reference would raise first while tracking."""
-        if nturns <= 0:
+        if nturns <= 0 or self.clean:
             return None
         order = list(range(start, end))
         if nturns > 1:
@@ -462,6 +459,7 @@ class CompiledLattice:
                 info.error = exc
         self.energy = energy
         self.rest_energy = rest_energy
+        self.clean = all(info.error is None for info in self.info)
 
 
 def _compile_element(el, idx: int, energy: float, rest_energy: float, t0: float,
@@ -519,10 +517,7 @@ def _compile_element(el, idx: int, energy: float, rest_energy: float, t0: float,
         rec.set(T.ATB_TM_ISCALE, _div(1.0, scaling))
         if scaling != 1.0:
             rec.flags |= T.ATB_F_SCALING
-        for i, v in enumerate(A):
-            rec.set(T.ATB_TM_POLY + i, v)
-        for i, v in enumerate(B):
-            rec.set(T.ATB_TM_POLY + mo + 1 + i, v)
+        rec.fields[T.ATB_TM_POLY:] = A + B
     elif op == T.ATB_OP_RFCAVITY:
         rec = _Record(op, T.ATB_RF_HALF + 1)
         le = _get_double(el, "Length")                  # RFCavityPass.c:367-373
@@ -633,7 +628,8 @@ def compile_lattice(line, energy: float = 0.0, rest_energy: float = 0.0,
         ring_length += element_length(el)
     if t0 is None:
         t0 = ring_length / C0
-    chunks = []
+    body: list[float] = []
+    headers: list[int] = []
     offsets = [0]
     infos: list[ElementInfo] = []
     efields: list[tuple[int, int, str]] = []
@@ -645,7 +641,10 @@ def compile_lattice(line, energy: float = 0.0, rest_energy: float = 0.0,
         try:
             rec = _compile_element(el, i, energy, rest_energy, t0, local, voltages,
                                    integrator)
-            w = rec.words()
+            h0, h1, n = rec.emit(body)
+            if n > T.ATB_MAX_RECORD_WORDS:
+                del body[pos:]
+                raise ValueError("element record too long (%d words)" % n)
             info = ElementInfo(op, pm, element_length(el), rec.max_order, rec.nsteps, rec.flags)
             if local and not energy > 0.0:
                 # RFCavityPass.c:376 / StrMPoleSymplectic4RadPass.c:148 refuse a
@@ -657,19 +656,23 @@ def compile_lattice(line, energy: float = 0.0, rest_energy: float = 0.0,
                 info.error = exc
         except (AttributeError, RuntimeError, ValueError, TypeError, KeyError, IndexError) as exc:
             local = []
-            w = _Record(T.ATB_OP_IDENTITY, 2).words()   # never executed
+            h0, h1, n = _Record(T.ATB_OP_IDENTITY, 2).emit(body)   # never executed
             info = ElementInfo(T.ATB_OP_IDENTITY, pm, element_length(el), error=exc)
         for (fw, _, kind) in local:
             efields.append((pos + fw, i, kind))
-        chunks.append(w)
+        headers.extend((h0, h1))
         infos.append(info)
-        pos += len(w)
+        pos += n
         offsets.append(pos)
-    words = np.concatenate(chunks) if chunks else np.zeros(0, dtype=np.float64)
+    words = np.array(body, dtype=np.float64)
+    u, at = words.view(np.uint64), np.asarray(offsets[:-1], dtype=np.int64)
+    u[at] = np.array(headers[0::2], dtype=np.uint64)
+    u[at + 1] = np.array(headers[1::2], dtype=np.uint64)
     cl = CompiledLattice(words=words, offsets=np.asarray(offsets, dtype=np.uint32),
                          info=infos, ring_length=ring_length, t0=t0, energy=energy,
                          rest_energy=rest_energy, charge=charge,
-                         energy_fields=efields, voltages=voltages)
+                         energy_fields=efields, voltages=voltages,
+                         clean=all(info.error is None for info in infos))
     return cl
 
 
