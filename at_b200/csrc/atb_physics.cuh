@@ -41,6 +41,12 @@ __device__ __forceinline__ double nan_d() { return __longlong_as_double(0x7ff800
 
 template <class T>
 __device__ __forceinline__ bool all_finite(const P6T<T>& r) {
+    if constexpr (!is_dual<T>::value) {
+        const uint32_t m = 0x7fffffffu;
+        const uint32_t a = max(max(rn_hi(r.x) & m, rn_hi(r.px) & m), rn_hi(r.y) & m);
+        const uint32_t b = max(max(rn_hi(r.py) & m, rn_hi(r.dp) & m), rn_hi(r.ct) & m);
+        return max(a, b) < 0x7ff00000u;
+    }
     return isfinite(val(r.x)) && isfinite(val(r.px)) && isfinite(val(r.y)) &&
            isfinite(val(r.py)) && isfinite(val(r.dp)) && isfinite(val(r.ct));
 }

@@ -82,11 +82,6 @@ ATB_RN_FN bool rn_within(double v, uint32_t lo_hi, uint32_t hi_hi) {
 ATB_RN_FN bool rn_below(double v, uint32_t hi_hi) {
     return (rn_hi(v) & 0x7fffffffu) < hi_hi;
 }
-/* a coordinate: zero, or 2^-400 <= |v| < 2^900 */
-ATB_RN_FN bool rn_coord_fits(double v) {
-    const uint32_t h = rn_hi(v) & 0x7fffffffu;
-    return h - 0x26f00000u < 0x78300000u - 0x26f00000u || (h | rn_lo(v)) == 0u;
-}
 /* 1 - 2^-53, the all-ones significand next to one */
 ATB_RN_FN bool rn_below_one(double v) {
     return rn_hi(v) == 0x3fefffffu && rn_lo(v) == 0xffffffffu;
@@ -100,14 +95,11 @@ ATB_RN_FN bool rn_near_fits(double d) {
 }
 /* a divisor of rn_rcp_nearer in [1, 1 + 2^-10) */
 ATB_RN_FN bool rn_nearer_fits(double d) { return rn_within(d, 0x3ff00000u, 0x3ff00400u); }
-/* a length: zero, or 2^-40 <= |v| < 2^40 */
-ATB_RN_FN bool rn_length_fits(double v) {
-    const uint32_t h = rn_hi(v) & 0x7fffffffu;
-    return h - 0x3d700000u < 0x42700000u - 0x3d700000u || (h | rn_lo(v)) == 0u;
-}
-/* The two tests of the step loops, where only tiny nonzero values are left to
-   exclude.  A denormal with a zero high word passes as zero; none comes up from
-   coordinates that passed rn_coord_fits. */
+/* What is left to exclude per particle are tiny nonzero values, whose
+   remainders or squares would underflow: two integer instructions each, zeros
+   passing.  A denormal below 2^-1042 has a zero high word and passes as well;
+   rn_denormal finds it where it would matter (a radiating kick's momenta: the
+   square of such a value is zero as it should be). */
 /* v >= 0: zero or at least 2^-860 */
 ATB_RN_FN bool rn_square_fits(double v) { return rn_hi(v) - 1u >= 0x0a300000u - 1u; }
 /* |v| zero or at least 2^-480 */
@@ -115,6 +107,15 @@ ATB_RN_FN bool rn_not_tiny(double v) {
     const uint32_t h = rn_hi(v);
     return h + h - 2u >= 2u * 0x21f00000u - 2u;
 }
+/* each of a magnet's entering coordinates zero or at least 2^-400 in size */
+ATB_RN_FN bool rn_coords_fit(double x, double px, double y, double py) {
+    const uint32_t a = 2u * rn_hi(x) - 2u, b = 2u * rn_hi(px) - 2u;
+    const uint32_t c = 2u * rn_hi(y) - 2u, d = 2u * rn_hi(py) - 2u;
+    const uint32_t ab = a < b ? a : b, cd = c < d ? c : d;
+    return (ab < cd ? ab : cd) >= 2u * 0x26f00000u - 2u;
+}
+/* nonzero with a zero high word */
+ATB_RN_FN bool rn_denormal(double v) { return 2u * rn_hi(v) == 0u && rn_lo(v) != 0u; }
 
 /* ---- arithmetic --------------------------------------------------------- */
 

@@ -73,6 +73,11 @@
 #define ATB_F_INTEG        (1u << 18)  /* thick multipole integrated by the
                                           integrator whose id (1-6) is stored at
                                           ATB_SM_INTEG, with step ATB_SM_SL */
+#define ATB_F_RN           (1u << 19)  /* thick multipole: the Forest-Ruth drift
+                                          lengths are zero or within 2^-39..2^39
+                                          and NumIntSteps at most 4096, where the
+                                          exact kernels' shared quotients hold
+                                          (without it they divide plainly)   */
 /* bend fringe "method" codes after host normalisation (atphyslib.c:15-79) */
 #define ATB_BM_LEGACY      0   /* method 0 or any value other than 1,2,3   */
 #define ATB_BM_1           1

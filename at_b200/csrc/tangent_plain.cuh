@@ -181,8 +181,7 @@ __device__ __forceinline__ void tan_steps(P6& r, TanCols& t, const Rec& e, const
     const P6 in = r;
     const double o = 1.0 + r.dp;
     const double od2 = 2.0 * o, hp = 0.5 * pb;
-    bool ok = rn_coord_fits(r.x) && rn_coord_fits(r.px) && rn_coord_fits(r.y) &&
-              rn_coord_fits(r.py) && rn_opd_fits(o) && rn_length_fits(nl1) && rn_length_fits(nl2);
+    bool ok = (e.flags() & ATB_F_RN) && rn_coords_fit(r.x, r.px, r.y, r.py) && rn_opd_fits(o);
     DriftInc d = fastdrift_inc(r, nl1, od2, hp, ok);
     tan_drift<DEC, HASK>(r, t, d, 1.0, nl1, pe, pb);
     add_drift(r, d);

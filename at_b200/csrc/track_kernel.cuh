@@ -134,23 +134,53 @@ struct Rec {
 
 /* ---------------- misalignment / aperture wrappers ----------------------- */
 
-template <class T>
+#define ATB_OPT_FIELD(slot) ((uint64_t)ATB_OPT_MASK << ((slot) * ATB_OPT_BITS))
+
+static __device__ __noinline__ P6 mult_dense_call(P6 r, const double* m) {
+    mult_dense(r, m);
+    return r;
+}
+static __device__ __noinline__ double apertures_call(P6 r, Rec e) {
+    if (const double* ra = e.blk(ATB_OPT_RAP)) check_rect(r, ra);
+    if (const double* ea = e.blk(ATB_OPT_EAP)) check_ellip(r, ea);
+    return r.ct;
+}
+
+/* CALL: the rare forms out of line */
+template <bool CALL = false, class T>
+__device__ __forceinline__ void misalign_rotation(P6T<T>& r, const double* m, bool dense) {
+    if constexpr (CALL) {
+        if (dense) r = mult_dense_call(r, m);
+        else mult_tilt(r, m);
+    } else {
+        mult_r(r, m, dense);
+    }
+}
+
+template <bool CALL = false, class T>
 __device__ __forceinline__ void entrance_misalign(P6T<T>& r, const Rec& e) {
     const uint32_t fl = e.flags();
     if (const double* t1 = e.blk(ATB_OPT_T1)) add_t(r, t1);
-    if (const double* r1 = e.blk(ATB_OPT_R1)) mult_r(r, r1, fl & ATB_F_R1_DENSE);
+    if (const double* r1 = e.blk(ATB_OPT_R1))
+        misalign_rotation<CALL>(r, r1, fl & ATB_F_R1_DENSE);
 }
 
-template <class T>
+template <bool CALL = false, class T>
 __device__ __forceinline__ void apertures(P6T<T>& r, const Rec& e) {
-    if (const double* ra = e.blk(ATB_OPT_RAP)) check_rect(r, ra);
-    if (const double* ea = e.blk(ATB_OPT_EAP)) check_ellip(r, ea);
+    if constexpr (CALL) {
+        if (e.opt & (ATB_OPT_FIELD(ATB_OPT_RAP) | ATB_OPT_FIELD(ATB_OPT_EAP)))
+            r.ct = apertures_call(r, e);
+    } else {
+        if (const double* ra = e.blk(ATB_OPT_RAP)) check_rect(r, ra);
+        if (const double* ea = e.blk(ATB_OPT_EAP)) check_ellip(r, ea);
+    }
 }
 
-template <class T>
+template <bool CALL = false, class T>
 __device__ __forceinline__ void exit_misalign(P6T<T>& r, const Rec& e) {
     const uint32_t fl = e.flags();
-    if (const double* r2 = e.blk(ATB_OPT_R2)) mult_r(r, r2, fl & ATB_F_R2_DENSE);
+    if (const double* r2 = e.blk(ATB_OPT_R2))
+        misalign_rotation<CALL>(r, r2, fl & ATB_F_R2_DENSE);
     if (const double* t2 = e.blk(ATB_OPT_T2)) add_t(r, t2);
 }
 
@@ -389,18 +419,17 @@ __device__ __forceinline__ void multipole_steps_rn(P6* r, Recip* c, const Rec& e
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         in[k] = r[k];
-        ok[k] = rn_coord_fits(r[k].x) && rn_coord_fits(r[k].px) && rn_coord_fits(r[k].y) &&
-                rn_coord_fits(r[k].py);
+        ok[k] = (e.flags() & ATB_F_RN) && rn_opd_fits(1.0 + r[k].dp) &&
+                rn_coords_fit(r[k].x, r[k].px, r[k].y, r[k].py);
     }
     if (RAD) {
         const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2), radc = e.f(ATB_SM_RADC);
-        const bool uniform = rn_length_fits(L1) && rn_length_fits(L2) && ns <= 4096;
         double o[NP], pn[NP];
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
             o[k] = 1.0 + r[k].dp;
             pn[k] = opd_rcp(c[k], r[k].dp);
-            ok[k] &= uniform && rn_opd_fits(o[k]);
+            ok[k] &= !rn_denormal(r[k].px) && !rn_denormal(r[k].py);
             d1[k] = drift_rad_inc(r[k], L1, pn[k]);
             add_drift_rad(r[k], d1[k]);
         }
@@ -442,8 +471,7 @@ __device__ __forceinline__ void multipole_steps_rn(P6* r, Recip* c, const Rec& e
             hp[k] = 0.5 * c[k].pn;
             /* the cached reciprocal is the entry's: an entrance shift may
                have changed delta since */
-            ok[k] &= rn_opd_fits(o) && r[k].dp == dp0[k] && rn_length_fits(nl1[k]) &&
-                     rn_length_fits(nl2[k]);
+            ok[k] &= r[k].dp == dp0[k];
             d1[k] = fastdrift_inc(r[k], nl1[k], od2[k], hp[k], ok[k]);
             add_drift(r[k], d1[k]);
         }
@@ -645,8 +673,10 @@ __device__ __forceinline__ void multipole_steps(P6T<T>* r, RecipOf<T>* c, const 
  * interleaves (NP = 2), while the element's parameters are read once.  Each
  * particle sees the same operations as alone (NP = 1).  The entrance and exit
  * are outside the choice of the step loop: one copy per pass method, which a
- * warp walking the lattice finds in the instruction cache. */
-template <int NP, bool BEND, bool RAD, bool GEN = false, class T>
+ * warp walking the lattice finds in the instruction cache.  LEAN: the form for
+ * elements without field scaling and quadrupole fringes, with dense rotations
+ * and apertures out of line. */
+template <int NP, bool BEND, bool RAD, bool GEN = false, bool LEAN = false, class T>
 __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const Rec& e,
                                                  const Param& pm) {
     const uint32_t fl = e.flags();
@@ -654,7 +684,7 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const
     T nl1[NP], nl2[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
-        if (fl & ATB_F_SCALING) change_pref<kFast>(r[k], e.f(ATB_SM_SCALE));
+        if (!LEAN && (fl & ATB_F_SCALING)) change_pref<kFast>(r[k], e.f(ATB_SM_SCALE));
         dp0[k] = val(r[k].dp);
         nl1[k] = 0.0;
         nl2[k] = 0.0;
@@ -664,8 +694,8 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const
             nl2[k] = e.f(ATB_SM_L2) * p_norm;
         }
         if (e.opt) {
-            entrance_misalign(r[k], e);
-            apertures(r[k], e);
+            entrance_misalign<LEAN>(r[k], e);
+            apertures<LEAN>(r[k], e);
         }
     }
     double irho = 0.0;
@@ -684,7 +714,7 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const
                                    1.0);
         }
     }
-    if (fl & ATB_F_FQ_IN) {
+    if (!LEAN && (fl & ATB_F_FQ_IN)) {
         const T b1 = fringe_b1<T>(e, pm);
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
@@ -699,7 +729,7 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const
         }
     }
     multipole_steps<NP, BEND, RAD, GEN>(r, c, e, pm, dp0, nl1, nl2, irho, e.nsteps());
-    if (fl & ATB_F_FQ_OUT) {
+    if (!LEAN && (fl & ATB_F_FQ_OUT)) {
         const T b1 = fringe_b1<T>(e, pm);
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
@@ -727,10 +757,10 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const
                                    fl & ATB_F_FC0_OUT, -1.0);
         }
         if (e.opt) {
-            apertures(r[k], e);
-            exit_misalign(r[k], e);
+            apertures<LEAN>(r[k], e);
+            exit_misalign<LEAN>(r[k], e);
         }
-        if (fl & ATB_F_SCALING) change_pref<kFast>(r[k], e.f(ATB_SM_ISCALE));
+        if (!LEAN && (fl & ATB_F_SCALING)) change_pref<kFast>(r[k], e.f(ATB_SM_ISCALE));
     }
 }
 
@@ -827,8 +857,6 @@ __device__ __forceinline__ void pass_corrector(P6T<T>& r, const Rec& e) {
     if (fl & ATB_F_SCALING) change_pref<kFast>(r, e.f(ATB_CO_ISCALE));
 }
 
-/* One element on one particle; lost particles (x is NaN) are skipped as every
- * reference pass method does (e.g. StrMPoleSymplectic4Pass.c:59). */
 /* QuantDiffPass.c: random kicks keyed by (key, pbase + p, nturn, ei);
  * without a key (the derivative kernels) the element is the identity, as the
  * reference's envelope code disables it */
@@ -845,11 +873,9 @@ __device__ __forceinline__ void pass_quantdiff(P6T<T>& r, const Rec& e, const At
 }
 
 template <bool GEN = false, class T>
-__device__ __forceinline__ void track_element(P6T<T>& r, RecipOf<T>& c, const Rec& e, int nturn,
-                                              const Param& pm = Param{-1, 0.0},
-                                              const AtbRng* rng = nullptr, long long p = 0,
-                                              int ei = 0) {
-    if (isnan(val(r.x))) return;
+__device__ __forceinline__ void track_element_any(P6T<T>& r, RecipOf<T>& c, const Rec& e,
+                                                  int nturn, const Param& pm, const AtbRng* rng,
+                                                  long long p, int ei) {
     switch (e.op()) {
         case ATB_OP_IDENTITY: pass_identity(r, e); break;
         case ATB_OP_DRIFT: pass_drift(r, c, e); break;
@@ -863,6 +889,58 @@ __device__ __forceinline__ void track_element(P6T<T>& r, RecipOf<T>& c, const Re
         case ATB_OP_APERTURE: check_rect(r, e.p + ATB_AP_LIM); break;
         case ATB_OP_QUANTDIFF: pass_quantdiff(r, e, rng, p, nturn, ei); break;
         default: break;
+    }
+}
+
+/* the same out of line */
+template <bool GEN>
+__device__ __noinline__ P6 track_element_call(P6 r, Rec e, int nturn, Param pm, const AtbRng* rng,
+                                              long long p, int ei) {
+    Recip c;
+    track_element_any<GEN>(r, c, e, nturn, pm, rng, p, ei);
+    return r;
+}
+
+/* One element on one particle; lost particles (x is NaN) are skipped as every
+ * reference pass method does (e.g. StrMPoleSymplectic4Pass.c:59).  Only what
+ * most of a lattice consists of is in line (CALL: drifts only): with cavities, correctors, thin
+ * multipoles, fringes and the rest beside them the particle moved between
+ * registers around every element (159 instructions for a drift, 14 of them
+ * FP64, where it now takes 88; a quadrupole beside its steps 1,060 cycles of a
+ * lone warp instead of 1,400). */
+template <bool GEN = false, bool CALL = false, class T>
+__device__ __forceinline__ void track_element(P6T<T>& r, RecipOf<T>& c, const Rec& e, int nturn,
+                                              const Param& pm = Param{-1, 0.0},
+                                              const AtbRng* rng = nullptr, long long p = 0,
+                                              int ei = 0) {
+    if (isnan(val(r.x))) return;
+    if constexpr (is_dual<T>::value) {
+        track_element_any<GEN>(r, c, e, nturn, pm, rng, p, ei);
+    } else {
+        const int op = e.op();
+        if (op == ATB_OP_DRIFT && e.opt == 0) {
+            drift6_pn<kFast>(r, e.f(ATB_DR_LE), opd_rcp(c, r.dp));
+            return;
+        }
+        if (!CALL && !(e.flags() & (ATB_F_SCALING | ATB_F_FQ_IN | ATB_F_FQ_OUT | ATB_F_INTEG))) {
+            if (op == ATB_OP_STRMPOLE) {
+                pass_multipole_n<1, false, false, false, true>(&r, &c, e, pm);
+                return;
+            }
+            if (op == ATB_OP_STRMPOLE_RAD) {
+                pass_multipole_n<1, false, true, false, true>(&r, &c, e, pm);
+                return;
+            }
+            if (op == ATB_OP_BNDMPOLE) {
+                pass_multipole_n<1, true, false, false, true>(&r, &c, e, pm);
+                return;
+            }
+            if (op == ATB_OP_BNDMPOLE_RAD) {
+                pass_multipole_n<1, true, true, false, true>(&r, &c, e, pm);
+                return;
+            }
+        }
+        r = track_element_call<GEN>(r, e, nturn, pm, rng, p, ei);
     }
 }
 
@@ -1270,12 +1348,12 @@ __device__ __forceinline__ void track_tiles(const AtbJob* __restrict__ jobs,
                     } else {
 #pragma unroll
                         for (int k = 0; k < NP; ++k)
-                            track_element<GEN>(r[k], rc[k], e, nturn[k], Param{-1, 0.0}, &J.rng,
-                                               p[k], ei);
+                            track_element<GEN, (NP > 1)>(r[k], rc[k], e, nturn[k],
+                                                         Param{-1, 0.0}, &J.rng, p[k], ei);
                     }
                     if (check_loss) {
 #pragma unroll
-                        for (int k = 0; k < NP; ++k)
+                        for (int k = 0; k < NP; ++k) {
                             if (losses ? !lost[k] && is_bad(r[k])
                                        : isfinite(r[k].x) && is_bad(r[k])) {
                                 if (losses && active[k])
@@ -1284,6 +1362,7 @@ __device__ __forceinline__ void track_tiles(const AtbJob* __restrict__ jobs,
                                 r[k].x = nan_d(); r[k].px = 0.0; r[k].y = 0.0;
                                 r[k].py = 0.0; r[k].dp = 0.0; r[k].ct = 0.0;
                             }
+                        }
                     }
                     w += e.len();
                 }

@@ -320,6 +320,9 @@ def _multipole_common(rec: _Record, el, op: int, bend: bool, integrator: int = 4
     rec.set(T.ATB_SM_L2, sl * DRIFT2)
     rec.set(T.ATB_SM_K1, sl * KICK1)
     rec.set(T.ATB_SM_K2, sl * KICK2)
+    if ns <= 4096 and all(v == 0.0 or 2.0 ** -39 <= v <= 2.0 ** 39
+                          for v in (abs(sl * DRIFT1), abs(sl * DRIFT2))):
+        rec.flags |= T.ATB_F_RN
     if integrator != 4:
         # another integrator of the GPU call: the step and the id replace the
         # Forest-Ruth lengths (atgpu/SymplecticIntegrator.cpp:140-171)

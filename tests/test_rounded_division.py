@@ -32,11 +32,14 @@ void nearer_(long n, const double* d, double* q, int* ok)
 void near_(long n, const double* d, double* q, int* ok)
 { for (long i = 0; i < n; ++i) { q[i] = rn_rcp_near(d[i]); ok[i] = rn_near_fits(d[i]); } }
 #define TEST_FN(name, f) void name(long n, const double* a, int* ok) \
-{ for (long i = 0; i < n; ++i) ok[i] = f(a[i]); }
-TEST_FN(coord_, rn_coord_fits)
-TEST_FN(length_, rn_length_fits)
-TEST_FN(square_, rn_square_fits)
-TEST_FN(tiny_, rn_not_tiny)
+{ for (long i = 0; i < n; ++i) ok[i] = f; }
+TEST_FN(square_, rn_square_fits(a[i]))
+TEST_FN(tiny_, rn_not_tiny(a[i]))
+TEST_FN(denormal_, rn_denormal(a[i]))
+TEST_FN(x_, rn_coords_fit(a[i], 1.0, 0.0, -1.0))
+TEST_FN(px_, rn_coords_fit(-0.0, a[i], 1.0, 1.0))
+TEST_FN(y_, rn_coords_fit(1.0, 0.0, a[i], 0.0))
+TEST_FN(py_, rn_coords_fit(0.0, 0.0, -1.0, a[i]))
 """
 
 
@@ -123,19 +126,29 @@ def test_reciprocals_equal_ieee_division(rn):
 
 
 def test_accepted_operands(rn):
-    """Each test's bounds; zeros pass, nothing else that is tiny does."""
-    for name, low, high in (("coord_", -400, 900), ("length_", -40, 40), ("square_", -860, None),
-                            ("tiny_", -480, None)):
+    """Each test's bound; zeros pass, nothing else that is tiny does except
+    denormals with a zero high word, which have a test of their own."""
+    for name, low in (("square_", -860), ("tiny_", -480), ("x_", -400), ("px_", -400),
+                      ("y_", -400), ("py_", -400)):
         lo = 2.0 ** low
-        a = np.array([0.0, 1.0, lo, np.nextafter(lo, 0.0), 2.0 ** -1040])
-        ok = [True, True, True, False, False]
+        a = np.array([0.0, 1.0, lo, np.nextafter(lo, 0.0), 2.0 ** -1040, 2.0 ** -1074])
+        ok = [True, True, True, False, False, True]
         if name != "square_":                       # the others take either sign
             a, ok = np.concatenate((a, -a)), ok + ok
-        if high is not None:                        # exact to the last denormal, bounded above
-            hi = 2.0 ** high
-            a = np.concatenate((a, [5e-324, np.nextafter(hi, 0.0), hi, np.inf, -np.inf, np.nan]))
-            ok = ok + [False, True, False, False, False, False]
         assert rn(name, a, flags=True, test=True).tolist() == ok, name
+    a = np.array([0.0, -0.0, 5e-324, -5e-324, 2.0 ** -1043, 2.0 ** -1042, 1.0, np.inf])
+    assert rn("denormal_", a, flags=True, test=True).tolist() == [
+        False, False, True, True, True, False, False, False]
+
+
+def test_table_flag_of_the_shared_quotients():
+    """ATB_F_RN: lengths within range and at most 4096 steps."""
+    from at_b200 import table as T
+    for length, ns, ok in ((0.4, 10, True), (0.0, 3, True), (-0.4, 4096, True), (0.4, 4097, False),
+                           (2.0 ** 45, 1, False), (2.0 ** -45, 1, False), (0.4, 0, False)):
+        el = E.Multipole("M", length, [0.0, 0.0], [0.0, 1.0], NumIntSteps=ns)
+        cl = compile_lattice([el], 3e9, ELECTRON_REST)
+        assert bool(cl.info[0].flags & T.ATB_F_RN) == ok, (length, ns)
 
 
 # -- on the GPU -----------------------------------------------------------------
