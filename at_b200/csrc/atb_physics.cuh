@@ -64,6 +64,23 @@ __device__ __forceinline__ double rcp_nr(double d) {
     return fma(y, e, y);
 }
 
+/* The same from what is known, in three or four fused operations and without
+ * the estimate (a trip to the XU pipe on the particle's chain): 1/o from the
+ * reciprocal y of a number within 2^-19 of it (a radiating kick changes
+ * 1 + delta by 1e-8), and 1/d of a number within 2^-9 of one; the series
+ * dropped are below 2^-54.  ok is cleared for anything else. */
+__device__ __forceinline__ double rcp_from(double o, double y, bool& ok) {
+    const double e = fma(-o, y, 1.0);
+    ok &= rn_below(e, 0x3ec00000u);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rcp_near_one(double d, bool& ok) {
+    const double y = 2.0 - d;
+    const double e = fma(-d, y, 1.0);
+    ok &= rn_within(d, 0x3feff000u, 0x3ff00800u);
+    return fma(y, fma(e, e, e), y);
+}
+
 /* atlalib.c:50-57 ATaddvv */
 template <class T>
 __device__ __forceinline__ void add_t(P6T<T>& r, const double* t) {
@@ -508,7 +525,8 @@ __device__ __forceinline__ void kick_rad_rn(P6T<double>& r, const PL& pl, double
  * ~1e-8 of delta), and (h_x + s/2)/(h_x^2 + s) in a bend.  The caller
  * converts px = x' opd, py = y' opd at the magnet's exit. */
 struct RadAngles {
-    double xp, yp, s, opd;
+    double xp, yp, s, opd, pn;      /* pn = 1/opd */
+    bool ok;                        /* the reciprocals' series held so far */
 };
 
 /* drift of length L, hL = L/2 */
@@ -520,23 +538,33 @@ __device__ __forceinline__ void rad_drift_fast(P6T<double>& r, RadAngles& a, dou
     r.ct = fma(hL, a.s, r.ct);
 }
 
-template <class PL>
+/* the same drift once more */
+__device__ __forceinline__ void rad_drift_again(P6T<double>& r, const RadAngles& a, double L,
+                                                double hL) {
+    r.x = fma(L, a.xp, r.x);
+    r.y = fma(L, a.yp, r.y);
+    r.ct = fma(hL, a.s, r.ct);
+}
+
+/* NR: with Newton-Raphson reciprocals, whatever the operands */
+template <bool NR, class PL>
 __device__ __forceinline__ void str_kick_rad_fast(P6T<double>& r, RadAngles& a, const PL& pl,
                                                   double L, double rL) {
     double re, im;
     pl.field(r.x, r.y, re, im);
-    const double g = a.s < 1e-5 ? fma(a.s, fma(0.5, a.s, -0.5), 1.0)
-                                : fma(0.5, a.s, 1.0) * rcp_nr(1.0 + a.s);
+    double g = fma(a.s, fma(0.5, a.s, -0.5), 1.0);
+    if (!NR) a.ok &= a.s < 1e-5;
+    else if (!(a.s < 1e-5)) g = fma(0.5, a.s, 1.0) * rcp_nr(1.0 + a.s);
     const double cr = fma(im, a.yp, -(re * a.xp));
     const double q = fma(re, re, fma(im, im, cr * cr));
     r.dp = fma(-(rL * q) * g, a.opd * a.opd, r.dp);
     a.opd = 1.0 + r.dp;
-    const double pn = rcp_nr(a.opd);
-    a.xp = fma(-L * re, pn, a.xp);
-    a.yp = fma(L * im, pn, a.yp);
+    a.pn = NR ? rcp_nr(a.opd) : rcp_from(a.opd, a.pn, a.ok);
+    a.xp = fma(-L * re, a.pn, a.xp);
+    a.yp = fma(L * im, a.pn, a.yp);
 }
 
-template <class PL>
+template <bool NR, class PL>
 __device__ __forceinline__ void bnd_kick_rad_fast(P6T<double>& r, RadAngles& a, const PL& pl,
                                                   double L, double irho, double lirho,
                                                   double rL) {
@@ -544,7 +572,7 @@ __device__ __forceinline__ void bnd_kick_rad_fast(P6T<double>& r, RadAngles& a, 
     pl.field(r.x, r.y, re, im);
     const double hx = fma(r.x, irho, 1.0);
     const double hx2 = hx * hx;
-    const double vn = rcp_nr(hx2 + a.s);
+    const double vn = NR ? rcp_nr(hx2 + a.s) : rcp_near_one(hx2 + a.s, a.ok);
     const double by = re + irho;
     const double cr = fma(im, a.yp, -(by * a.xp));
     const double q = fma(fma(by, by, im * im), hx2, cr * cr);
@@ -552,10 +580,10 @@ __device__ __forceinline__ void bnd_kick_rad_fast(P6T<double>& r, RadAngles& a, 
     const double dp0 = r.dp;
     r.dp = fma(-(rL * q) * (h * vn), a.opd * a.opd, r.dp);
     a.opd = 1.0 + r.dp;
-    const double pn = rcp_nr(a.opd);
+    a.pn = NR ? rcp_nr(a.opd) : rcp_from(a.opd, a.pn, a.ok);
     const double u = fma(-fma(-r.x, irho, dp0), irho, re);
-    a.xp = fma(-L * u, pn, a.xp);
-    a.yp = fma(L * im, pn, a.yp);
+    a.xp = fma(-L * u, a.pn, a.xp);
+    a.yp = fma(L * im, a.pn, a.yp);
     r.ct = fma(lirho, r.x, r.ct);
 }
 
