@@ -24,6 +24,7 @@ ATB_ERR_NOLAT = -5
 MODE_EXACT = 0
 MODE_FAST = 1
 FLAG_ELEMENT = 1
+FLAG_ZEROED = 2
 
 _lock = threading.Lock()
 _lib = None

@@ -164,6 +164,8 @@ struct atb_handle {
     cudaEvent_t launched = nullptr;    /* the last launch that uses the handle's lists */
     char* stage[2] = {nullptr, nullptr};            /* pinned snapshot staging */
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+    cudaStream_t copies = nullptr;                  /* snapshots on their way back */
+    cudaEvent_t tracked = nullptr;                  /* a chunk's snapshots are there */
 };
 
 /* The serving loop: a persistent kernel that claims tiles from a queue the
@@ -600,6 +602,8 @@ int atb_destroy(atb_handle* h) {
             if (h->stage[i]) cudaFreeHost(h->stage[i]);
             if (h->stage_ev[i]) cudaEventDestroy(h->stage_ev[i]);
         }
+        if (h->copies) cudaStreamDestroy(h->copies);
+        if (h->tracked) cudaEventDestroy(h->tracked);
         if (h->launched) cudaEventDestroy(h->launched);
         if (h->stream) cudaStreamDestroy(h->stream);
     }
@@ -747,13 +751,59 @@ namespace {
 
 constexpr int64_t kStageBytes = 64LL << 20;   /* each of the two staging buffers */
 constexpr int64_t kStageDirect = 8LL << 20;   /* smaller copies go directly      */
+constexpr int64_t kStagePiped = 16LL << 20;   /* larger ones overlap the tracking */
+
+int ensure_staging(atb_handle* h) {
+    for (int i = 0; i < 2; ++i) {
+        if (!h->stage[i])
+            ATB_CUDA(cudaHostAlloc((void**)&h->stage[i], (size_t)kStageBytes, cudaHostAllocDefault));
+        if (!h->stage_ev[i])
+            ATB_CUDA(cudaEventCreateWithFlags(&h->stage_ev[i], cudaEventDisableTiming));
+    }
+    return ATB_OK;
+}
+
+/* Device bytes [off, off + len) of snapshots whose slots are `row` bytes each,
+   in the staging buffer, to slots `pitch` bytes apart from dst, by several
+   host threads: the caller's fresh (not yet touched) pages cost one thread
+   more time than the copy. */
+void place_snapshots(const char* stage, char* dst, int64_t off, int64_t len, int64_t row,
+                     int64_t pitch) {
+    const int nthr = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    /* device bytes [b0, b1) of this piece to their rows of rout */
+    auto place = [=](int64_t b0, int64_t b1) {
+        if (pitch == row) {              /* all particles: one block */
+            std::memcpy(dst + b0, stage + (b0 - off), (size_t)(b1 - b0));
+            return;
+        }
+        while (b0 < b1) {
+            const int64_t slot = b0 / row, within = b0 - slot * row;
+            const int64_t n = std::min(b1 - b0, row - within);
+            std::memcpy(dst + slot * pitch + within, stage + (b0 - off), (size_t)n);
+            b0 += n;
+        }
+    };
+    const int64_t part = (len + nthr - 1) / nthr;
+    std::vector<std::thread> th;
+    for (int t = 1; t < nthr; ++t) {
+        const int64_t b0 = off + std::min<int64_t>(len, t * part);
+        const int64_t b1 = off + std::min<int64_t>(len, (t + 1) * part);
+        if (b0 >= b1) continue;
+        try {
+            th.emplace_back(place, b0, b1);
+        } catch (...) {
+            place(b0, b1);     /* no thread to be had: this one does it */
+        }
+    }
+    place(off, off + std::min<int64_t>(len, part));
+    for (std::thread& x : th) x.join();
+}
 
 /* The snapshots of one chunk -- `slots` slots of gn particles, gn * 48 bytes
    each, contiguous on the device -- to slots [slot0, slot0 + slots) of the
    caller's rout (np particles a slot), columns [a, a + gn).  Small copies go
    directly; large ones through two pinned staging buffers: the GPU fills one
-   while host threads place the other, so the copy is not held to one
-   thread's pace through the caller's fresh (not yet touched) pages. */
+   while host threads place the other. */
 int copy_snapshots(atb_handle* h, cudaStream_t st, const double* dev, int64_t slots, int64_t gn,
                    double* rout, int64_t np, int64_t a, int64_t slot0) {
     const int64_t row = gn * 48, pitch = np * 48, total = slots * row;
@@ -766,12 +816,8 @@ int copy_snapshots(atb_handle* h, cudaStream_t st, const double* dev, int64_t sl
                                        (size_t)slots, cudaMemcpyDeviceToHost, st));
         return ATB_OK;
     }
-    for (int i = 0; i < 2; ++i) {
-        if (!h->stage[i])
-            ATB_CUDA(cudaHostAlloc((void**)&h->stage[i], (size_t)kStageBytes, cudaHostAllocDefault));
-        if (!h->stage_ev[i])
-            ATB_CUDA(cudaEventCreateWithFlags(&h->stage_ev[i], cudaEventDisableTiming));
-    }
+    int rc = ensure_staging(h);
+    if (rc) return rc;
     const char* src = reinterpret_cast<const char*>(dev);
     const int64_t npieces = (total + kStageBytes - 1) / kStageBytes;
     auto issue = [&](int64_t p) {
@@ -780,39 +826,11 @@ int copy_snapshots(atb_handle* h, cudaStream_t st, const double* dev, int64_t sl
                                         cudaMemcpyDeviceToHost, st);
         return e == cudaSuccess ? cudaEventRecord(h->stage_ev[p & 1], st) : e;
     };
-    const int nthr = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
     for (int64_t p = 0; p < std::min<int64_t>(2, npieces); ++p) ATB_CUDA(issue(p));
     for (int64_t p = 0; p < npieces; ++p) {
         ATB_CUDA(cudaEventSynchronize(h->stage_ev[p & 1]));
         const int64_t off = p * kStageBytes, len = std::min(kStageBytes, total - off);
-        const char* stage = h->stage[p & 1];
-        /* device bytes [b0, b1) of this piece to their rows of rout */
-        auto place = [=](int64_t b0, int64_t b1) {
-            if (pitch == row) {              /* all particles: one block */
-                std::memcpy(dst + b0, stage + (b0 - off), (size_t)(b1 - b0));
-                return;
-            }
-            while (b0 < b1) {
-                const int64_t slot = b0 / row, within = b0 - slot * row;
-                const int64_t n = std::min(b1 - b0, row - within);
-                std::memcpy(dst + slot * pitch + within, stage + (b0 - off), (size_t)n);
-                b0 += n;
-            }
-        };
-        const int64_t part = (len + nthr - 1) / nthr;
-        std::vector<std::thread> th;
-        for (int t = 1; t < nthr; ++t) {
-            const int64_t b0 = off + std::min<int64_t>(len, t * part);
-            const int64_t b1 = off + std::min<int64_t>(len, (t + 1) * part);
-            if (b0 >= b1) continue;
-            try {
-                th.emplace_back(place, b0, b1);
-            } catch (...) {
-                place(b0, b1);     /* no thread to be had: this one does it */
-            }
-        }
-        place(off, off + std::min<int64_t>(len, part));
-        for (std::thread& x : th) x.join();
+        place_snapshots(h->stage[p & 1], dst, off, len, row, pitch);
         if (p + 2 < npieces) ATB_CUDA(issue(p + 2));   /* into the buffer just placed */
     }
     return ATB_OK;
@@ -889,10 +907,23 @@ int atb_track(atb_handle* h, int32_t id, double* rin, int64_t np, int32_t nturns
     int64_t turns_per_chunk = nturns;
     if (nref > 0 && rec_turn > 0)
         turns_per_chunk = std::max<int64_t>(1, h->rout_budget / (rec_turn * slot_bytes));
+    /* Snapshots of some size come back while the next turns are tracked: at
+       least four chunks of turns, none larger than a staging buffer, each in
+       its own part of the device buffer (10,007 particles x 10 turns of the
+       FODO ring with 32 points, 154 MB: 12.8 -> @MON@ ms). */
+    const int64_t turn_bytes = rec_max * slot_bytes;
+    const bool piped = nref > 0 && group == np && nturns > 1 && turns_per_chunk >= nturns &&
+                       turn_bytes > 0 && turn_bytes <= kStageBytes &&
+                       nturns * turn_bytes > kStagePiped;
+    const int64_t region = piped ? rec_first + (nturns - 1) * rec_turn : 0;   /* slots */
+    if (piped)
+        turns_per_chunk = std::max<int64_t>(
+            1, std::min<int64_t>((nturns + 3) / 4, kStageBytes / turn_bytes));
     /* the first chunk holds rec_first + (nt - 1) rec_turn slots, the others
        nt rec_turn, nt <= turns_per_chunk: within the budget */
     const int64_t max_slots =
-        nref ? std::max<int64_t>(
+        piped ? region
+        : nref ? std::max<int64_t>(
                    rec_first + (std::min<int64_t>(turns_per_chunk, nturns) - 1) * rec_turn,
                    turns_per_chunk * rec_turn)
              : 0;
@@ -906,6 +937,38 @@ int atb_track(atb_handle* h, int32_t id, double* rin, int64_t np, int32_t nturns
     bool gen = false;
     int rc = kernel_config(h, lats, mode, &smem, &grid_max, &gen);
     if (rc) return rc;
+
+    if (piped) {
+        rc = ensure_staging(h);
+        if (rc) return rc;
+        if (!h->copies) ATB_CUDA(cudaStreamCreateWithFlags(&h->copies, cudaStreamNonBlocking));
+        if (!h->tracked)
+            ATB_CUDA(cudaEventCreateWithFlags(&h->tracked, cudaEventDisableTiming));
+    }
+    /* a piped chunk whose snapshots are in a staging buffer (or on their way)
+       and not yet placed */
+    struct Pending {
+        int64_t off, bytes;
+        int buf;
+    };
+    std::vector<Pending> pending;
+    int next_buf = 0;
+    /* no return leaves a copy in flight */
+    struct Drain {
+        cudaStream_t st;
+        ~Drain() {
+            if (st) cudaStreamSynchronize(st);
+        }
+    } drain{piped ? h->copies : nullptr};
+    auto place_first = [&]() -> cudaError_t {
+        const Pending q = pending.front();
+        pending.erase(pending.begin());
+        const cudaError_t e = cudaEventSynchronize(h->stage_ev[q.buf]);
+        if (e == cudaSuccess)
+            place_snapshots(h->stage[q.buf], reinterpret_cast<char*>(rout), q.off, q.bytes,
+                            slot_bytes, slot_bytes);
+        return e;
+    };
 
     for (int64_t a = 0; a < np; a += group) {
         const int64_t gn = std::min<int64_t>(group, np - a);
@@ -926,7 +989,7 @@ int atb_track(atb_handle* h, int32_t id, double* rin, int64_t np, int32_t nturns
             J.nref = nref;
             J.losses = losses ? 1 : 0;
             J.rout = nref ? h->rout.as<double>() : nullptr;
-            J.rout_slot0 = 0;
+            J.rout_slot0 = piped ? slot_done : 0;
             J.lost = losses ? h->lost.as<uint8_t>() + a : nullptr;
             J.lturn = losses ? h->lturn.as<uint32_t>() + a : nullptr;
             J.lelem = losses ? h->lelem.as<uint32_t>() + a : nullptr;
@@ -942,6 +1005,21 @@ int atb_track(atb_handle* h, int32_t id, double* rin, int64_t np, int32_t nturns
             if (rc) return rc;
             if (nref) {
                 int64_t slots = (t0 == 0 ? rec_first : rec_turn) + (int64_t)(nt - 1) * rec_turn;
+                if (piped) {
+                    /* a buffer is free again once the chunk before last is placed */
+                    if (pending.size() == 2) ATB_CUDA(place_first());
+                    const Pending q{slot_done * slot_bytes, slots * slot_bytes, next_buf};
+                    slot_done += slots;
+                    if (q.bytes == 0) continue;
+                    next_buf ^= 1;
+                    ATB_CUDA(cudaEventRecord(h->tracked, st));
+                    ATB_CUDA(cudaStreamWaitEvent(h->copies, h->tracked, 0));
+                    ATB_CUDA(cudaMemcpyAsync(h->stage[q.buf], h->rout.as<char>() + q.off,
+                                             (size_t)q.bytes, cudaMemcpyDeviceToHost, h->copies));
+                    ATB_CUDA(cudaEventRecord(h->stage_ev[q.buf], h->copies));
+                    pending.push_back(q);
+                    continue;
+                }
                 if (slots > 0) {
                     rc = copy_snapshots(h, st, h->rout.as<double>(), slots, gn, rout, np, a,
                                         slot_done);
@@ -954,12 +1032,22 @@ int atb_track(atb_handle* h, int32_t id, double* rin, int64_t np, int32_t nturns
             ATB_CUDA(cudaStreamSynchronize(st));
         }
     }
+    while (!pending.empty()) ATB_CUDA(place_first());
     ATB_CUDA(cudaMemcpyAsync(rin, h->r.p, rbytes, cudaMemcpyDeviceToHost, st));
     if (losses) {
         ATB_CUDA(cudaMemcpyAsync(islost, h->lost.p, np, cudaMemcpyDeviceToHost, st));
-        ATB_CUDA(cudaMemcpyAsync(lturn, h->lturn.p, np * 4, cudaMemcpyDeviceToHost, st));
-        ATB_CUDA(cudaMemcpyAsync(lelem, h->lelem.p, np * 4, cudaMemcpyDeviceToHost, st));
-        ATB_CUDA(cudaMemcpyAsync(lcoord, h->lcoord.p, rbytes, cudaMemcpyDeviceToHost, st));
+        /* where nothing was lost the rest of the map is zeros, which the caller
+           may hold already: 56 bytes a particle of fresh pages stay untouched */
+        bool write = true;
+        if (flags & ATB_FLAG_ZEROED) {
+            ATB_CUDA(cudaStreamSynchronize(st));
+            write = std::memchr(islost, 1, (size_t)np) != nullptr;
+        }
+        if (write) {
+            ATB_CUDA(cudaMemcpyAsync(lturn, h->lturn.p, np * 4, cudaMemcpyDeviceToHost, st));
+            ATB_CUDA(cudaMemcpyAsync(lelem, h->lelem.p, np * 4, cudaMemcpyDeviceToHost, st));
+            ATB_CUDA(cudaMemcpyAsync(lcoord, h->lcoord.p, rbytes, cudaMemcpyDeviceToHost, st));
+        }
     }
     if (alive) ATB_CUDA(cudaMemcpyAsync(alive, h->alive.p, (size_t)nturns * 4, cudaMemcpyDeviceToHost, st));
     if (moments)

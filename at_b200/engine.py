@@ -142,7 +142,7 @@ class Engine:
                 int(end_elem), ptr(refs) if nref else None, nref,
                 ptr(rout) if (nref and npart) else None, 1 if losses else 0, ptr(islost),
                 ptr(lturn), ptr(lelem), ptr(lcoord), ptr(alive), ptr(moments), mode_code(mode),
-                _lib.FLAG_ELEMENT if element else 0))
+                (_lib.FLAG_ELEMENT if element else 0) | _lib.FLAG_ZEROED))
         if losses:
             ld = {"islost": islost, "turn": lturn, "elem": lelem, "coord": lcoord}
         return rout, ld, ((alive, moments) if stats else None)

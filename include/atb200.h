@@ -45,6 +45,8 @@ extern "C" {
 #define ATB_MODE_FAST 1       /* FMA + reciprocal reuse                    */
 
 #define ATB_FLAG_ELEMENT 1    /* single-element pass: no loss marking      */
+#define ATB_FLAG_ZEROED 2     /* the caller's loss-map arrays hold zeros: they
+                                 are not written when nothing was lost     */
 
 typedef struct atb_handle atb_handle;
 
