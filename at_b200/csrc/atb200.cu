@@ -910,7 +910,7 @@ int atb_track(atb_handle* h, int32_t id, double* rin, int64_t np, int32_t nturns
     /* Snapshots of some size come back while the next turns are tracked: at
        least four chunks of turns, none larger than a staging buffer, each in
        its own part of the device buffer (10,007 particles x 10 turns of the
-       FODO ring with 32 points, 154 MB: 12.8 -> @MON@ ms). */
+       FODO ring with 32 points, 154 MB: 12.8 -> 9.3 ms). */
     const int64_t turn_bytes = rec_max * slot_bytes;
     const bool piped = nref > 0 && group == np && nturns > 1 && turns_per_chunk >= nturns &&
                        turn_bytes > 0 && turn_bytes <= kStageBytes &&

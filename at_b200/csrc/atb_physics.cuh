@@ -553,7 +553,7 @@ __device__ __forceinline__ void str_kick_rad_fast(P6T<double>& r, RadAngles& a, 
     double re, im;
     pl.field(r.x, r.y, re, im);
     double g = fma(a.s, fma(0.5, a.s, -0.5), 1.0);
-    if (!NR) a.ok &= a.s < 1e-5;
+    if (!NR) a.ok &= rn_below(a.s, 0x3ee00000u);       /* 2^-17, by its exponent */
     else if (!(a.s < 1e-5)) g = fma(0.5, a.s, 1.0) * rcp_nr(1.0 + a.s);
     const double cr = fma(im, a.yp, -(re * a.xp));
     const double q = fma(re, re, fma(im, im, cr * cr));

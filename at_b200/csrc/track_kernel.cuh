@@ -578,7 +578,7 @@ __device__ __forceinline__ void rad_steps_fast(P6* r, Recip* c, const Rec& e, co
         a[k] = RadAngles{r[k].px * pn, r[k].py * pn, 0.0, 1.0 + r[k].dp, pn, true};
         rad_drift_fast(r[k], a[k], L1, h1);
     }
-    for (int m = 1; m <= ns; ++m) {
+    for (int m = 1;; ++m) {
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
             if (BEND) bnd_kick_rad_fast<NR>(r[k], a[k], pl, K1, irho, k1i, rk1);
@@ -599,10 +599,10 @@ __device__ __forceinline__ void rad_steps_fast(P6* r, Recip* c, const Rec& e, co
             else str_kick_rad_fast<NR>(r[k], a[k], pl, K1, rk1);
         }
 #pragma unroll
-        for (int k = 0; k < NP; ++k) {
-            rad_drift_fast(r[k], a[k], L1, h1);
-            if (m < ns) rad_drift_again(r[k], a[k], L1, h1);
-        }
+        for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L1, h1);
+        if (m == ns) break;
+#pragma unroll
+        for (int k = 0; k < NP; ++k) rad_drift_again(r[k], a[k], L1, h1);
     }
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
@@ -620,7 +620,7 @@ __device__ __noinline__ P6 rad_steps_fast_call(P6 r, Rec e, Param pm) {
     pl.load(A, A + mo + 1, mo);
     if (pm.k >= 0) pl.set_param(pm.k, pm.v);
     Recip c;
-    bool ok[1];
+    bool ok[1];               /* called for at least one step */
     rad_steps_fast<1, BEND, true>(&r, &c, e, pl, BEND ? e.f(ATB_BM_IRHO) : 0.0, e.nsteps(), ok);
     return r;
 }
@@ -628,14 +628,14 @@ __device__ __noinline__ P6 rad_steps_fast_call(P6 r, Rec e, Param pm) {
 /* The fast kernels' steps.  A radiating magnet in which an operand leaves the
  * range of the reciprocals' series is tracked again with Newton-Raphson ones
  * (a branch at each would cut the kicks into blocks: 24.5 ms for 300,000
- * particles and a turn of the large ring against 20.3 and, with Newton-Raphson
+ * particles and a turn of the large ring against 19.9 and, with Newton-Raphson
  * throughout, 21.3). */
 template <int NP, bool BEND, bool RAD, class PL>
 __device__ __forceinline__ void multipole_steps_fast(P6* r, Recip* c, const Rec& e, const PL& pl,
                                                      const Param& pm, const double* nl1,
                                                      const double* nl2, double irho, int ns) {
+    if (ns <= 0) return;
     if (RAD) {
-        if (ns <= 0) return;
         P6 in[NP];
         bool ok[NP];
 #pragma unroll
