@@ -18,9 +18,8 @@
  * going to a scratch array ([element][particle][6], coalesced) -- or the
  * forward pass stored every turn's (memory permitting); then
  * atb_adjoint_turn_kernel walks the elements backwards with
- * lambda <- J_e^T lambda, J_e
- * the element's Jacobian at its stored entry state, and at an element that
- * carries K_q, dL/dK_q += (d r_out / d K_q) . lambda_out, summed over the
+ * lambda <- J_e^T lambda, J_e the element's Jacobian at its stored entry
+ * state, and at an element that carries K_q, dL/dK_q += (d r_out / d K_q) . lambda_out, summed over the
  * block's particles in shared memory and added to the global sum once per
  * block.
  *
@@ -36,16 +35,17 @@
  *    field derivative F'(z) of F(z) = sum (B_n + i A_n) z^n from a second
  *    Horner recursion and dF/dB_k = z^k for the strength.
  *  - every other element (radiating magnets, quadrupole fringes, field
- *    scaling, thick correctors, bend edges of method 3): J_e from a forward-mode evaluation of the whole element on dual
- *    numbers (6 directions, 7 when the element carries a strength), out of
- *    line so that its registers do not weigh on the common path.
+ *    scaling, thick correctors, bend edges of method 3): J_e from a
+ *    forward-mode evaluation of the whole element on dual numbers (6
+ *    directions, 7 when the element carries a strength), out of line so that
+ *    its registers do not weigh on the common path.
  * A particle that is lost (NaN, or lost during the turn) gets a NaN
  * cotangent and adds nothing to the strengths' gradient.
  *
  * Bound by dependent FP64 latency at 3.5 warps a scheduler (65,536 particles).
  * A turn of the FODO ring with 128 strengths backwards: 5.0 ms with the step
- * entries recomputed into shared memory and every step run twice more; 2.4 ms
- * with the stages undone from the exit (1.0 of it the tracking), which needs
+ * entries recomputed into shared memory and every step run twice more; 2.3 ms
+ * with the stages undone from the exit (0.9 of it the tracking), which needs
  * no store and keeps one stage's coordinates instead of seven.
  */
 #ifndef ATB_ADJOINT_KERNEL_CUH

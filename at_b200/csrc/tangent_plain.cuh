@@ -15,8 +15,8 @@
  *
  * Bound: the FP64 pipe when the SMs are full, dependent latency below that
  * (one warp a scheduler up to 19,000 particles).  One turn of the FODO ring with
- * 128 strengths: 16,411 particles 1.62 ms (4.6 on dual numbers), 65,536
- * particles 3.74 ms (12.9).  168 registers and three blocks an SM: with 128
+ * 128 strengths: 16,411 particles 1.50 ms (4.6 on dual numbers), 65,536
+ * particles 3.72 ms (12.9).  168 registers and three blocks an SM: with 128
  * and four the columns spill (3 KB of stores), with 255 and two the larger set
  * takes 3.85 ms.
  */

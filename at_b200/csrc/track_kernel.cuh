@@ -160,7 +160,7 @@ __device__ __forceinline__ void misalign_rotation(P6T<T>& r, const double* m, bo
 /* The usual misalignment, a shift and a rotation of the x/y planes: one branch,
  * and the fourteen words (16-byte aligned blocks) asked for at once.  One by
  * one, each branch waited for its own words: 375 cycles a warp and magnet with
- * 16 warps on an SM, 213 so. */
+ * 16 warps on an SM, 172 so. */
 struct ShiftTilt {
     double2 t[3], m[4];
 };
@@ -444,8 +444,8 @@ __device__ __noinline__ P6 multipole_steps_call(P6 r, Rec e, Param pm, double nl
  * The divisions bounded these loops: about nine FP64 instructions each, a
  * seed on the XU pipe and a branch to a slow path that ended the block the
  * compiler could interleave (a plain sextupole step of a lone warp took 631
- * cycles and takes 275, a radiating one 1886 and 958; of 16 warps a scheduler
- * each takes 296 and now 174 cycles a plain step, 836 and 495 a radiating
+ * cycles and takes 275, a radiating one 1886 and 946; of 16 warps a scheduler
+ * each takes 296 and now 160 cycles a plain step, 836 and 498 a radiating
  * one).  The last drift of a step and the
  * first of the next have the same length, momenta and 1/(1+delta), hence the
  * same increments: they are computed once and added twice.  A warp with an
