@@ -125,6 +125,7 @@ struct Batch {
     DevBuf jobs, tiles, counter, scratch, jobnext;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    cudaEvent_t launched = nullptr;    /* the last launch of these lists */
 };
 
 struct Lattice {
@@ -162,6 +163,7 @@ struct atb_handle {
     std::vector<AtbTile> h_tiles;
     std::vector<struct Batch> batches;
     cudaEvent_t launched = nullptr;    /* the last launch that uses the handle's lists */
+    cudaEvent_t derived = nullptr;     /* the last that uses the tan_, adj_ buffers */
     char* stage[2] = {nullptr, nullptr};            /* pinned snapshot staging */
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};
     cudaStream_t copies = nullptr;                  /* snapshots on their way back */
@@ -340,22 +342,36 @@ int kernel_config(atb_handle* h, const std::vector<const Lattice*>& lats, int mo
     return ATB_OK;
 }
 
+/* Memory that belongs to the handle or to a prepared batch -- launch lists,
+   counters, strength maps, scratch -- is shared by every stream: work that
+   writes it waits for the event of the last work that used it, whatever
+   stream that was on, and leaves the event for the next, on every way out.
+   (Inside a stream capture there is nothing to wait for or to record.) */
+struct InOrder {
+    cudaEvent_t event = nullptr;
+    cudaStream_t st = nullptr;
+    cudaError_t begin(cudaEvent_t& last, cudaStream_t stream) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(stream, &cap);
+        if (e != cudaSuccess || cap != cudaStreamCaptureStatusNone) return e;
+        if (!last) e = cudaEventCreateWithFlags(&last, cudaEventDisableTiming);
+        else e = cudaStreamWaitEvent(stream, last, 0);
+        if (e != cudaSuccess) return e;
+        event = last;
+        st = stream;
+        return cudaSuccess;
+    }
+    ~InOrder() {
+        if (event) cudaEventRecord(event, st);
+    }
+};
+
 int launch(atb_handle* h, const std::vector<AtbJob>& jobs, const std::vector<AtbTile>& tiles,
            int smem_bytes, int grid_max, int mode, cudaStream_t st, int threads, int ppt,
            bool gen) {
     if (tiles.empty()) return ATB_OK;
-    /* The launch lists, counters and scratch belong to the handle: a launch on
-       another stream waits for the last one before it replaces them.  (Inside
-       a stream capture there is nothing to wait for or to record.) */
-    cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
-    ATB_CUDA(cudaStreamIsCapturing(st, &cap_st));
-    const bool ordered = cap_st == cudaStreamCaptureStatusNone;
-    if (ordered) {
-        if (!h->launched)
-            ATB_CUDA(cudaEventCreateWithFlags(&h->launched, cudaEventDisableTiming));
-        else
-            ATB_CUDA(cudaStreamWaitEvent(st, h->launched, 0));
-    }
+    InOrder in_order;
+    ATB_CUDA(in_order.begin(h->launched, st));
     if (h->jobs.ensure(jobs.size() * sizeof(AtbJob)) != cudaSuccess ||
         h->tiles.ensure(tiles.size() * sizeof(AtbTile)) != cudaSuccess)
         return fail(ATB_ERR_CUDA, "cudaMalloc(launch lists) failed");
@@ -400,7 +416,6 @@ int launch(atb_handle* h, const std::vector<AtbJob>& jobs, const std::vector<Atb
         atb_track_kernel_fast<<<grid, threads, smem_bytes, st>>>(dj, dt, nt, cnt, jn, sts, cap,
                                                                  scr);
     ATB_CUDA(cudaGetLastError());
-    if (ordered) ATB_CUDA(cudaEventRecord(h->launched, st));
     return ATB_OK;
 }
 
@@ -590,6 +605,7 @@ int atb_destroy(atb_handle* h) {
             B.counter.release();
             B.scratch.release();
             B.jobnext.release();
+            if (B.launched) cudaEventDestroy(B.launched);
         }
         for (DevBuf* b : {&h->r, &h->rout, &h->lost, &h->lturn, &h->lelem, &h->lcoord,
                           &h->refpts, &h->jobs, &h->tiles, &h->counter, &h->status, &h->alive,
@@ -605,6 +621,7 @@ int atb_destroy(atb_handle* h) {
         if (h->copies) cudaStreamDestroy(h->copies);
         if (h->tracked) cudaEventDestroy(h->tracked);
         if (h->launched) cudaEventDestroy(h->launched);
+        if (h->derived) cudaEventDestroy(h->derived);
         if (h->stream) cudaStreamDestroy(h->stream);
     }
     delete h;
@@ -1229,7 +1246,11 @@ int atb_tangent_device(atb_handle* h, int32_t id, double* r, int64_t np, int32_t
     A.nparam = nparam;
     A.r = r;
     A.np = np;
+    const long long blocks = (np + ATB_TANGENT_THREADS - 1) / ATB_TANGENT_THREADS;
+    if (blocks > 0x7fffffffLL) return fail(ATB_ERR_ARG, "too many particles");
+    InOrder in_order;
     if (nparam > 0) {
+        ATB_CUDA(in_order.begin(h->derived, st));
         if (h->tan_pelem.ensure(h->h_pelem.size() * 4) != cudaSuccess ||
             h->tan_porder.ensure((size_t)nparam * 4) != cudaSuccess)
             return fail(ATB_ERR_NOMEM, "cudaMalloc(parameter map) failed");
@@ -1245,8 +1266,6 @@ int atb_tangent_device(atb_handle* h, int32_t id, double* r, int64_t np, int32_t
     A.jac = jac;
     A.grad = grad;
     A.lost = islost;
-    const long long blocks = (np + ATB_TANGENT_THREADS - 1) / ATB_TANGENT_THREADS;
-    if (blocks > 0x7fffffffLL) return fail(ATB_ERR_ARG, "too many particles");
     if (tangent_by_hand(*L))
         atb_tangent_plain_kernel<<<(unsigned)blocks, ATB_TANGENT_THREADS, 0, st>>>(A);
     else
@@ -1305,6 +1324,8 @@ int atb_adjoint_forward(atb_handle* h, int32_t id, double* r, int64_t np, int32_
     DeviceGuard g(h->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : h->stream;
     AtbAdjoint A;
+    InOrder in_order;
+    if (nparam > 0) ATB_CUDA(in_order.begin(h->derived, st));
     const int rs = adjoint_setup(h, L, param_order, param_value, nparam, st, A);
     if (rs != ATB_OK) return rs;
     A.nturns = nturns;
@@ -1347,6 +1368,8 @@ int atb_adjoint_backward(atb_handle* h, int32_t id, const double* ckpt, int64_t 
     if (nparam > 0) ATB_CUDA(cudaMemsetAsync(gparam, 0, (size_t)nparam * sizeof(double), st));
     if (np == 0 || nturns == 0) return ATB_OK;
     AtbAdjoint A;
+    InOrder in_order;
+    if (nparam > 0 || !estates) ATB_CUDA(in_order.begin(h->derived, st));
     const int rs = adjoint_setup(h, L, param_order, param_value, nparam, st, A);
     if (rs != ATB_OK) return rs;
     const size_t smem = (size_t)nparam * sizeof(double);
@@ -1643,6 +1666,8 @@ int atb_batch_launch(atb_handle* h, int32_t batch_id, void* stream) {
     if (!B) return fail(ATB_ERR_ARG, "unknown batch id");
     DeviceGuard g(h->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : h->stream;
+    InOrder in_order;
+    ATB_CUDA(in_order.begin(B->launched, st));
     if (B->exec) {
         ATB_CUDA(cudaGraphLaunch(B->exec, st));
         return ATB_OK;
@@ -1665,6 +1690,8 @@ int atb_batch_free(atb_handle* h, int32_t batch_id) {
     B->counter.release();
     B->scratch.release();
     B->jobnext.release();
+    if (B->launched) cudaEventDestroy(B->launched);
+    B->launched = nullptr;
     B->used = false;
     return ATB_OK;
 }
