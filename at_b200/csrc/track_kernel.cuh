@@ -304,7 +304,7 @@ __device__ __forceinline__ void multipole_steps_generic(P6T<T>* r, const Rec& e,
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 const double pn = 1.0 / (1.0 + r[k].dp);
-                a[k] = RadAngles{r[k].px * pn, r[k].py * pn, 0.0, 1.0 + r[k].dp, pn, true};
+                a[k] = RadAngles{r[k].px * pn, r[k].py * pn, 0.0, 1.0 + r[k].dp};
             }
             for (int m = 0; m < ns; ++m) {
                 for (int i = 0; i < ig.n; ++i) {
@@ -317,8 +317,8 @@ __device__ __forceinline__ void multipole_steps_generic(P6T<T>* r, const Rec& e,
                         const double lk = SL * ig.d[i];
 #pragma unroll
                         for (int k = 0; k < NP; ++k) {
-                            if (BEND) bnd_kick_rad_fast<true>(r[k], a[k], pl, lk, irho, lk * irho, radc * lk);
-                            else str_kick_rad_fast<true>(r[k], a[k], pl, lk, radc * lk);
+                            if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, lk, irho, lk * irho, radc * lk);
+                            else str_kick_rad_fast(r[k], a[k], pl, lk, radc * lk);
                         }
                     }
                 }
@@ -561,12 +561,11 @@ __device__ __forceinline__ void multipole_steps_rn(P6* r, Recip* c, const Rec& e
         }
 }
 
-/* The fast kernels' radiating steps, NR: with Newton-Raphson reciprocals.  A
- * step's last drift and the first of the next share angles and increments.
- * Returns whether the reciprocals' series held. */
-template <int NP, bool BEND, bool NR, class PL>
+/* The fast kernels' radiating steps.  A step's last drift and the first of
+ * the next share angles and increments. */
+template <int NP, bool BEND, class PL>
 __device__ __forceinline__ void rad_steps_fast(P6* r, Recip* c, const Rec& e, const PL& pl,
-                                               double irho, int ns, bool (&ok)[NP]) {
+                                               double irho, int ns) {
     const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
     const double k1i = BEND ? e.f(ATB_BM_K1IRHO) : 0.0, k2i = BEND ? e.f(ATB_BM_K2IRHO) : 0.0;
     const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2), radc = e.f(ATB_SM_RADC);
@@ -575,28 +574,28 @@ __device__ __forceinline__ void rad_steps_fast(P6* r, Recip* c, const Rec& e, co
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         const double pn = opd_rcp(c[k], r[k].dp);
-        a[k] = RadAngles{r[k].px * pn, r[k].py * pn, 0.0, 1.0 + r[k].dp, pn, true};
+        a[k] = RadAngles{r[k].px * pn, r[k].py * pn, 0.0, 1.0 + r[k].dp};
         rad_drift_fast(r[k], a[k], L1, h1);
     }
     for (int m = 1;; ++m) {
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
-            if (BEND) bnd_kick_rad_fast<NR>(r[k], a[k], pl, K1, irho, k1i, rk1);
-            else str_kick_rad_fast<NR>(r[k], a[k], pl, K1, rk1);
+            if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K1, irho, k1i, rk1);
+            else str_kick_rad_fast(r[k], a[k], pl, K1, rk1);
         }
 #pragma unroll
         for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L2, h2);
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
-            if (BEND) bnd_kick_rad_fast<NR>(r[k], a[k], pl, K2, irho, k2i, rk2);
-            else str_kick_rad_fast<NR>(r[k], a[k], pl, K2, rk2);
+            if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K2, irho, k2i, rk2);
+            else str_kick_rad_fast(r[k], a[k], pl, K2, rk2);
         }
 #pragma unroll
         for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L2, h2);
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
-            if (BEND) bnd_kick_rad_fast<NR>(r[k], a[k], pl, K1, irho, k1i, rk1);
-            else str_kick_rad_fast<NR>(r[k], a[k], pl, K1, rk1);
+            if (BEND) bnd_kick_rad_fast(r[k], a[k], pl, K1, irho, k1i, rk1);
+            else str_kick_rad_fast(r[k], a[k], pl, K1, rk1);
         }
 #pragma unroll
         for (int k = 0; k < NP; ++k) rad_drift_fast(r[k], a[k], L1, h1);
@@ -608,42 +607,17 @@ __device__ __forceinline__ void rad_steps_fast(P6* r, Recip* c, const Rec& e, co
     for (int k = 0; k < NP; ++k) {
         r[k].px = a[k].xp * a[k].opd;
         r[k].py = a[k].yp * a[k].opd;
-        ok[k] = a[k].ok;
     }
 }
 
-template <bool BEND>
-__device__ __noinline__ P6 rad_steps_fast_call(P6 r, Rec e, Param pm) {
-    const int mo = e.mo();
-    const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
-    Poly<-1> pl;
-    pl.load(A, A + mo + 1, mo);
-    if (pm.k >= 0) pl.set_param(pm.k, pm.v);
-    Recip c;
-    bool ok[1];               /* called for at least one step */
-    rad_steps_fast<1, BEND, true>(&r, &c, e, pl, BEND ? e.f(ATB_BM_IRHO) : 0.0, e.nsteps(), ok);
-    return r;
-}
-
-/* The fast kernels' steps.  A radiating magnet in which an operand leaves the
- * range of the reciprocals' series is tracked again with Newton-Raphson ones
- * (a branch at each would cut the kicks into blocks: 24.5 ms for 300,000
- * particles and a turn of the large ring against 19.9 and, with Newton-Raphson
- * throughout, 21.3). */
+/* The fast kernels' steps. */
 template <int NP, bool BEND, bool RAD, class PL>
 __device__ __forceinline__ void multipole_steps_fast(P6* r, Recip* c, const Rec& e, const PL& pl,
-                                                     const Param& pm, const double* nl1,
-                                                     const double* nl2, double irho, int ns) {
+                                                     const double* nl1, const double* nl2,
+                                                     double irho, int ns) {
     if (ns <= 0) return;
     if (RAD) {
-        P6 in[NP];
-        bool ok[NP];
-#pragma unroll
-        for (int k = 0; k < NP; ++k) in[k] = r[k];
-        rad_steps_fast<NP, BEND, false>(r, c, e, pl, irho, ns, ok);
-#pragma unroll
-        for (int k = 0; k < NP; ++k)
-            if (!ok[k]) r[k] = rad_steps_fast_call<BEND>(in[k], e, pm);
+        rad_steps_fast<NP, BEND>(r, c, e, pl, irho, ns);
     } else {
         const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
         const double k1i = BEND ? e.f(ATB_BM_K1IRHO) : 0.0, k2i = BEND ? e.f(ATB_BM_K2IRHO) : 0.0;
@@ -690,7 +664,7 @@ __device__ __forceinline__ void multipole_steps_mo(P6* r, Recip* c, const Rec& e
     Poly<MO, SKEW> pl;
     pl.load(A, A + mo + 1, mo);
     if (pm.k >= 0) pl.set_param(pm.k, pm.v);
-    if constexpr (kFast) multipole_steps_fast<NP, BEND, RAD>(r, c, e, pl, pm, nl1, nl2, irho, ns);
+    if constexpr (kFast) multipole_steps_fast<NP, BEND, RAD>(r, c, e, pl, nl1, nl2, irho, ns);
     else multipole_steps_rn<NP, BEND, RAD>(r, c, e, pl, pm, dp0, nl1, nl2, irho, ns);
 }
 
