@@ -668,7 +668,7 @@ __device__ __forceinline__ void multipole_steps_mo(P6* r, Recip* c, const Rec& e
     else multipole_steps_rn<NP, BEND, RAD>(r, c, e, pl, pm, dp0, nl1, nl2, irho, ns);
 }
 
-template <int NP, bool BEND, bool RAD, bool GEN, class T>
+template <int NP, bool BEND, bool RAD, bool INTEG, class T>
 __device__ __forceinline__ void multipole_steps(P6T<T>* r, RecipOf<T>* c, const Rec& e,
                                                 const Param& pm, const double* dp0, const T* nl1,
                                                 const T* nl2, double irho, int ns) {
@@ -680,24 +680,16 @@ __device__ __forceinline__ void multipole_steps(P6T<T>* r, RecipOf<T>* c, const 
         pl.load(A, A + mo + 1, mo);
         if (pm.k >= 0) pl.set_param(pm.k, pm.v);
         multipole_steps_plain<NP, BEND, RAD>(r, e, pl, nl1, nl2, irho, ns);
+    } else if constexpr (INTEG) {
+        /* another integrator of the GPU call: steps of SL*c[i] drift and
+           SL*d[i] kick (atgpu/SymplecticIntegrator.cpp:140-171) */
+        const int mo = e.mo();
+        const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
+        Poly<-1> pl;
+        pl.load(A, A + mo + 1, mo);
+        if (pm.k >= 0) pl.set_param(pm.k, pm.v);
+        multipole_steps_generic<NP, BEND, RAD>(r, e, pl, nl2, irho, ns);
     } else {
-        /* tables compiled for another integrator of the GPU call take one
-           generic instance, in the kernels built with them (GEN); the hosts
-           of the other kernels send them none (atb_track_noalloc checks its
-           raw table with a scan kernel, the tangent host refuses it) */
-        if constexpr (GEN) {
-            if (e.flags() & ATB_F_INTEG) {
-                const int mo = e.mo();
-                const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
-                Poly<-1> pl;
-                pl.load(A, A + mo + 1, mo);
-                if (pm.k >= 0) pl.set_param(pm.k, pm.v);
-                /* steps of SL*c[i] drift and SL*d[i] kick
-                   (atgpu/SymplecticIntegrator.cpp:140-171) */
-                multipole_steps_generic<NP, BEND, RAD>(r, e, pl, nl2, irho, ns);
-                return;
-            }
-        }
 #define ATB_STEPS(MO, SKEW) \
     multipole_steps_mo<NP, MO, BEND, RAD, SKEW>(r, c, e, pm, dp0, nl1, nl2, irho, ns)
         /* upright magnets' fields without the zero skew terms */
@@ -733,7 +725,7 @@ __device__ __forceinline__ void multipole_steps(P6T<T>* r, RecipOf<T>* c, const 
  * warp walking the lattice finds in the instruction cache.  LEAN: the form for
  * elements without field scaling and quadrupole fringes, with dense rotations
  * and apertures out of line. */
-template <int NP, bool BEND, bool RAD, bool GEN = false, bool LEAN = false, class T>
+template <int NP, bool BEND, bool RAD, bool INTEG = false, bool LEAN = false, class T>
 __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const Rec& e,
                                                  const Param& pm) {
     const uint32_t fl = e.flags();
@@ -785,7 +777,7 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const
             }
         }
     }
-    multipole_steps<NP, BEND, RAD, GEN>(r, c, e, pm, dp0, nl1, nl2, irho, e.nsteps());
+    multipole_steps<NP, BEND, RAD, INTEG>(r, c, e, pm, dp0, nl1, nl2, irho, e.nsteps());
     if (!LEAN && (fl & ATB_F_FQ_OUT)) {
         const T b1 = fringe_b1<T>(e, pm);
 #pragma unroll
@@ -929,17 +921,17 @@ __device__ __forceinline__ void pass_quantdiff(P6T<T>& r, const Rec& e, const At
     }
 }
 
-template <bool GEN = false, class T>
+template <class T>
 __device__ __forceinline__ void track_element_any(P6T<T>& r, RecipOf<T>& c, const Rec& e,
                                                   int nturn, const Param& pm, const AtbRng* rng,
                                                   long long p, int ei) {
     switch (e.op()) {
         case ATB_OP_IDENTITY: pass_identity(r, e); break;
         case ATB_OP_DRIFT: pass_drift(r, c, e); break;
-        case ATB_OP_STRMPOLE: pass_multipole_n<1, false, false, GEN>(&r, &c, e, pm); break;
-        case ATB_OP_STRMPOLE_RAD: pass_multipole_n<1, false, true, GEN>(&r, &c, e, pm); break;
-        case ATB_OP_BNDMPOLE: pass_multipole_n<1, true, false, GEN>(&r, &c, e, pm); break;
-        case ATB_OP_BNDMPOLE_RAD: pass_multipole_n<1, true, true, GEN>(&r, &c, e, pm); break;
+        case ATB_OP_STRMPOLE: pass_multipole_n<1, false, false>(&r, &c, e, pm); break;
+        case ATB_OP_STRMPOLE_RAD: pass_multipole_n<1, false, true>(&r, &c, e, pm); break;
+        case ATB_OP_BNDMPOLE: pass_multipole_n<1, true, false>(&r, &c, e, pm); break;
+        case ATB_OP_BNDMPOLE_RAD: pass_multipole_n<1, true, true>(&r, &c, e, pm); break;
         case ATB_OP_THINMPOLE: pass_thinmpole(r, e, pm); break;
         case ATB_OP_RFCAVITY: pass_rfcavity(r, e, nturn); break;
         case ATB_OP_CORRECTOR: pass_corrector(r, e); break;
@@ -950,12 +942,24 @@ __device__ __forceinline__ void track_element_any(P6T<T>& r, RecipOf<T>& c, cons
 }
 
 /* the same out of line */
-template <bool GEN>
-__device__ __noinline__ P6 track_element_call(P6 r, Rec e, int nturn, Param pm, const AtbRng* rng,
-                                              long long p, int ei) {
+static __device__ __noinline__ P6 track_element_call(P6 r, Rec e, int nturn, Param pm,
+                                                     const AtbRng* rng, long long p, int ei) {
     Recip c;
-    track_element_any<GEN>(r, c, e, nturn, pm, rng, p, ei);
+    track_element_any(r, c, e, nturn, pm, rng, p, ei);
     return r;
+}
+
+/* A magnet of a table compiled for another integrator of the GPU call, in the
+ * kernels built with them (GEN); the hosts of the other kernels send them none
+ * (atb_track_noalloc checks its raw table with a scan kernel, the tangent host
+ * refuses it). */
+__device__ __forceinline__ void track_integ(P6& r, Recip& c, const Rec& e, const Param& pm) {
+    switch (e.op()) {
+        case ATB_OP_STRMPOLE: pass_multipole_n<1, false, false, true>(&r, &c, e, pm); break;
+        case ATB_OP_STRMPOLE_RAD: pass_multipole_n<1, false, true, true>(&r, &c, e, pm); break;
+        case ATB_OP_BNDMPOLE: pass_multipole_n<1, true, false, true>(&r, &c, e, pm); break;
+        default: pass_multipole_n<1, true, true, true>(&r, &c, e, pm); break;
+    }
 }
 
 /* One element on one particle; lost particles (x is NaN) are skipped as every
@@ -972,14 +976,22 @@ __device__ __forceinline__ void track_element(P6T<T>& r, RecipOf<T>& c, const Re
                                               int ei = 0) {
     if (isnan(val(r.x))) return;
     if constexpr (is_dual<T>::value) {
-        track_element_any<GEN>(r, c, e, nturn, pm, rng, p, ei);
+        track_element_any(r, c, e, nturn, pm, rng, p, ei);
     } else {
         const int op = e.op();
         if (op == ATB_OP_DRIFT && e.opt == 0) {
             drift6_pn<kFast>(r, e.f(ATB_DR_LE), opd_rcp(c, r.dp));
             return;
         }
-        if (!CALL && !(e.flags() & (ATB_F_SCALING | ATB_F_FQ_IN | ATB_F_FQ_OUT | ATB_F_INTEG))) {
+        if constexpr (GEN) {
+            /* in line: out of line their coefficients, read on every kick, come
+               through generic addresses, 3 to 9 % slower on full SMs */
+            if (e.flags() & ATB_F_INTEG) {
+                track_integ(r, c, e, pm);
+                return;
+            }
+        }
+        if (!CALL && !(e.flags() & (ATB_F_SCALING | ATB_F_FQ_IN | ATB_F_FQ_OUT))) {
             if (op == ATB_OP_STRMPOLE) {
                 pass_multipole_n<1, false, false, false, true>(&r, &c, e, pm);
                 return;
@@ -997,7 +1009,7 @@ __device__ __forceinline__ void track_element(P6T<T>& r, RecipOf<T>& c, const Re
                 return;
             }
         }
-        r = track_element_call<GEN>(r, e, nturn, pm, rng, p, ei);
+        r = track_element_call(r, e, nturn, pm, rng, p, ei);
     }
 }
 
