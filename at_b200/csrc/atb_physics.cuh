@@ -416,12 +416,11 @@ __device__ __forceinline__ void diff_drift_pn(P6T<T>& r, double L, const T& pn) 
 
 /* The exact kernels' forms of the drift and the radiating kicks, on doubles:
  * the expressions above with their divisions taken from the reciprocals at
- * hand (atb_rn.h), the same IEEE results without a seed, a range test or a
- * slow branch per division.  `ok` is cleared when an operand leaves the range
- * in which that holds (tiny numerators, angles above 31 mrad or a path factor
- * further than 2^-8 from one, an energy loss above 2^-20 in one kick, anything
- * not finite), tested on exponents with integer instructions; the caller then
- * tracks the magnet again by the plain expressions. */
+ * hand (atb_rn.h), the same IEEE results without a range test or a slow
+ * branch per division.  What they need is tested once a magnet, at its entry
+ * (1 + delta) and at its exit (the largest energy loss of a kick, nothing tiny
+ * and everything finite); a magnet that fails is tracked by the plain
+ * expressions.  Angles and the distance from the axis have no bound. */
 
 /* what a drift adds to x, y and ct (to ct twice that in a radiating magnet,
  * whose drift halves the last product: ct + w/2 is one fused operation, w/2
@@ -442,9 +441,8 @@ __device__ __forceinline__ void add_drift_rad(P6T<double>& r, const DriftInc& d)
 
 /* fastdrift: od2 = 2(1 + delta), hp = RN(1/(1 + delta))/2 */
 __device__ __forceinline__ DriftInc fastdrift_inc(const P6T<double>& r, double nl, double od2,
-                                                  double hp, bool& ok) {
+                                                  double hp) {
     const double s = r.px * r.px + r.py * r.py;
-    ok &= rn_square_fits(s);
     return DriftInc{nl * r.px, nl * r.py, rn_div(nl * s, od2, hp)};
 }
 
@@ -459,14 +457,14 @@ __device__ __forceinline__ DriftInc drift_rad_inc(const P6T<double>& r, double L
 template <bool BEND, class PL>
 __device__ __forceinline__ void kick_rad_rn(P6T<double>& r, const PL& pl, double L, double irho,
                                             double lirho, double radc, double& o, double& pn,
-                                            bool& ok) {
+                                            uint32_t& loss) {
     double re, im;
     pl.field(r.x, r.y, re, im);
     const double xpr = r.px * pn, ypr = r.py * pn;
     const double xx = xpr * xpr, yy = ypr * ypr;
     const double hx = BEND ? 1.0 + r.x * irho : 1.0;
     const double d = (BEND ? hx * hx + xx : 1.0 + xx) + yy;
-    const double v_norm2 = BEND ? rn_rcp_near(d) : rn_rcp_nearer(d);
+    const double v_norm2 = rn_rcp_near(d);
     const double bx = im, by = BEND ? re + irho : re;
     const double cr = bx * ypr - by * xpr;
     double b2p;
@@ -480,9 +478,8 @@ __device__ __forceinline__ void kick_rad_rn(P6T<double>& r, const PL& pl, double
     r.dp -= radc * b2p * factor;
     o = 1.0 + r.dp;
     double e;
-    pn = rn_rcp_from(o, pn, &e);
-    ok &= (BEND ? rn_near_fits(d) : rn_nearer_fits(d)) && rn_below(e, ATB_RN_SEED_HI) &&
-          !rn_below_one(o) && rn_not_tiny(xpr) && rn_not_tiny(ypr);
+    pn = BEND ? rn_rcp_from_wide(o, pn, &e) : rn_rcp_from(o, pn, &e);
+    loss = max(loss, rn_hi(e) & 0x7fffffffu);
     r.px = rn_div(xpr, pn, o);
     r.py = rn_div(ypr, pn, o);
     if (BEND) {

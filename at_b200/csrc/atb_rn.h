@@ -31,8 +31,11 @@
  * The remainder is exact, or the quotient lies more than an ulp and less than
  * one and a half from q0, where rounding it in its last bit changes nothing.
  * A reciprocal's last step, y + y (1 - d y), is exact for y next to 1/d unless
- * d's significand is all ones (Markstein); for d near one that is the single
- * number 1 - u, which the callers exclude.
+ * d's significand is all ones (Markstein).  There 1/d lies just above the
+ * midpoint of its neighbours and the step from the upper one is right, from
+ * the lower one wrong, so the y before it is rounded upwards (rn_fma_up).
+ * That may leave y an ulp and a little above 1/d where 1/d is within 2^-54 of
+ * a double: far from any midpoint, and the step is right again.
  * No step may underflow or overflow: the callers bound the operands and send
  * everything else through the plain divisions.
  *
@@ -42,6 +45,7 @@
 #ifndef ATB_RN_H
 #define ATB_RN_H
 
+#include <fenv.h>
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
@@ -86,20 +90,21 @@ ATB_RN_FN bool rn_below(double v, uint32_t hi_hi) {
 ATB_RN_FN bool rn_below_one(double v) {
     return rn_hi(v) == 0x3fefffffu && rn_lo(v) == 0xffffffffu;
 }
-/* 1 + delta within 7/64 of one: 4096 steps of three kicks that each change it
-   by 2^-20 at most leave it in [7/8, 9/8) */
-ATB_RN_FN bool rn_opd_fits(double o) { return rn_within(o, 0x3fec8000u, 0x3ff1c000u); }
-/* a divisor of rn_rcp_near in [1 - 2^-8, 1 + 2^-8) */
-ATB_RN_FN bool rn_near_fits(double d) {
-    return rn_within(d, 0x3fefe000u, 0x3ff01000u) && !rn_below_one(d);
-}
-/* a divisor of rn_rcp_nearer in [1, 1 + 2^-10) */
-ATB_RN_FN bool rn_nearer_fits(double d) { return rn_within(d, 0x3ff00000u, 0x3ff00400u); }
+/* 1 + delta in a magnet without radiation, in [1/2, 2) */
+ATB_RN_FN bool rn_opd_constant(double o) { return rn_within(o, 0x3fe00000u, 0x40000000u); }
+/* 1 + delta at the entry of a radiating magnet, in [97/128, 5/4): the kicks
+   that rn_rcp_from and rn_rcp_from_wide accept (3 x 4096 of 2^-18, 3 x 256 of
+   2^-14) leave it in (0.7072, 1.4141), where its square and that of its
+   reciprocal are between 1/2 and 2 */
+ATB_RN_FN bool rn_opd_fits(double o) { return rn_within(o, 0x3fe84000u, 0x3ff40000u); }
+/* divisors of rn_rcp_near: normal, below 2^1000 */
+ATB_RN_FN bool rn_near_fits(double d) { return rn_within(d, 0x00100000u, 0x7e700000u); }
+/* the same of divisors known to be at least 1 */
+ATB_RN_FN bool rn_nearer_fits(double d) { return rn_within(d, 0x3ff00000u, 0x7e700000u); }
 /* What is left to exclude per particle are tiny nonzero values, whose
    remainders or squares would underflow: two integer instructions each, zeros
    passing.  A denormal below 2^-1042 has a zero high word and passes as well;
-   rn_denormal finds it where it would matter (a radiating kick's momenta: the
-   square of such a value is zero as it should be). */
+   rn_denormal finds it where it would matter. */
 /* v >= 0: zero or at least 2^-860 */
 ATB_RN_FN bool rn_square_fits(double v) { return rn_hi(v) - 1u >= 0x0a300000u - 1u; }
 /* |v| zero or at least 2^-480 */
@@ -116,6 +121,14 @@ ATB_RN_FN bool rn_coords_fit(double x, double px, double y, double py) {
 }
 /* nonzero with a zero high word */
 ATB_RN_FN bool rn_denormal(double v) { return 2u * rn_hi(v) == 0u && rn_lo(v) != 0u; }
+/* zero or at least 2^-480 in size, and below 2^400: what a magnet's exit is
+   tested for.  A quotient of values below 2^-960 may be wrong in its last
+   bits.  Added to anything of ordinary size it vanishes in the rounding,
+   whichever bits it has; where it does not, the sum is as tiny, and is found
+   here at the exit. */
+ATB_RN_FN bool rn_ordinary(double v) {
+    return rn_not_tiny(v) && !rn_denormal(v) && rn_below(v, 0x58f00000u);
+}
 
 /* ---- arithmetic --------------------------------------------------------- */
 
@@ -129,27 +142,60 @@ ATB_RN_FN double rn_div(double a, double b, double y) {
 /* one Newton step of the reciprocal of d */
 ATB_RN_FN double rn_rcp_step(double d, double y) { return fma(fma(-d, y, 1.0), y, y); }
 
-/* RN(1 / o) from the reciprocal `seed` of a neighbouring number; e = 1 - o seed
-   must be below 2^-20 (the series drops e^3) and o not 1 - 2^-53 */
+/* a b + c rounded upwards */
+ATB_RN_FN double rn_fma_up(double a, double b, double c) {
+#ifdef __CUDA_ARCH__
+    return __fma_ru(a, b, c);
+#else
+    volatile double x = a, r;
+    const int mode = fegetround();
+    fesetround(FE_UPWARD);
+    r = fma(x, b, c);
+    fesetround(mode);
+    return r;
+#endif
+}
+
+/* RN(1 / o) from the reciprocal `seed` of a neighbouring number: e = 1 - o seed
+   must be below 2^-18, or 2^-14 with a term more (the series drop e^3 and e^4) */
 ATB_RN_FN double rn_rcp_from(double o, double seed, double* e) {
     const double d = fma(-o, seed, 1.0);
     *e = d;
-    return rn_rcp_step(o, fma(seed, fma(d, d, d), seed));
+    return rn_rcp_step(o, rn_fma_up(seed, fma(d, d, d), seed));
 }
-#define ATB_RN_SEED_HI 0x3eb00000u   /* 2^-20 */
+#define ATB_RN_SEED_HI 0x3ed00000u   /* 2^-18 */
+ATB_RN_FN double rn_rcp_from_wide(double o, double seed, double* e) {
+    const double d = fma(-o, seed, 1.0);
+    *e = d;
+    return rn_rcp_step(o, rn_fma_up(seed, fma(fma(d, d, d), d, d), seed));
+}
+/* its bound, by the steps that 1 + delta has to stay in range for */
+ATB_RN_FN uint32_t rn_seed_wide_hi(int nsteps) {
+    return nsteps <= 256 ? 0x3f100000u : ATB_RN_SEED_HI;   /* 2^-14 */
+}
 
-/* RN(1 / d) for d within 2^-8 of one, from 2 - d: its residue (d - 1)^2 in a
-   geometric series to the third power, to the second for d within 2^-10 */
-ATB_RN_FN double rn_rcp_nearer(double d) {
-    const double y = 2.0 - d;
-    const double r = fma(-d, y, 1.0);
-    return rn_rcp_step(d, fma(y, fma(r, r, r), y));
+/* 1 / d to 20 bits (on the host, for the tests, the quotient's high word) */
+ATB_RN_FN double rn_estimate(double d) {
+    double y;
+#ifdef __CUDA_ARCH__
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+#else
+    uint64_t b;
+    y = 1.0 / d;
+    memcpy(&b, &y, 8);
+    b &= 0xffffffff00000000ull;
+    memcpy(&y, &b, 8);
+#endif
+    return y;
 }
+
+/* RN(1 / d): the estimate's residue in a geometric series to the second power
+   (the third is below 2^-54 for an estimate of 18 bits), then the exact step */
 ATB_RN_FN double rn_rcp_near(double d) {
-    const double y = 2.0 - d;
+    const double y = rn_estimate(d);
     const double r = fma(-d, y, 1.0);
-    const double t = fma(fma(r, r, r), r, r);
-    return rn_rcp_step(d, fma(y, t, y));
+    return rn_rcp_step(d, rn_fma_up(y, fma(r, r, r), y));
 }
+ATB_RN_FN double rn_rcp_nearer(double d) { return rn_rcp_near(d); }
 
 #endif /* ATB_RN_H */

@@ -181,8 +181,8 @@ __device__ __forceinline__ void tan_steps(P6& r, TanCols& t, const Rec& e, const
     const P6 in = r;
     const double o = 1.0 + r.dp;
     const double od2 = 2.0 * o, hp = 0.5 * pb;
-    bool ok = (e.flags() & ATB_F_RN) && rn_coords_fit(r.x, r.px, r.y, r.py) && rn_opd_fits(o);
-    DriftInc d = fastdrift_inc(r, nl1, od2, hp, ok);
+    bool ok = (e.flags() & ATB_F_RN) && rn_coords_fit(r.x, r.px, r.y, r.py) && rn_opd_constant(o);
+    DriftInc d = fastdrift_inc(r, nl1, od2, hp);
     tan_drift<DEC, HASK>(r, t, d, 1.0, nl1, pe, pb);
     add_drift(r, d);
     for (int m = 1;; ++m) {
@@ -191,19 +191,19 @@ __device__ __forceinline__ void tan_steps(P6& r, TanCols& t, const Rec& e, const
             const double K = h ? K2 : K1, ki = h ? k2i : k1i;
             tan_kick<DEC, BEND, HASK>(r, t, pl, pm.k, K, irho, ki);
             if (BEND) bndthinkick(r, pl, K, irho, ki); else strthinkick(r, pl, K);
-            d = fastdrift_inc(r, nl2, od2, hp, ok);
+            d = fastdrift_inc(r, nl2, od2, hp);
             tan_drift<DEC, HASK>(r, t, d, 1.0, nl2, pe, pb);
             add_drift(r, d);
         }
         tan_kick<DEC, BEND, HASK>(r, t, pl, pm.k, K1, irho, k1i);
         if (BEND) bndthinkick(r, pl, K1, irho, k1i); else strthinkick(r, pl, K1);
-        d = fastdrift_inc(r, nl1, od2, hp, ok);
+        d = fastdrift_inc(r, nl1, od2, hp);
         tan_drift<DEC, HASK>(r, t, d, m == ns ? 1.0 : 2.0, nl1, pe, pb);
         add_drift(r, d);
         if (m == ns) break;
         add_drift(r, d);
     }
-    ok &= rn_below(r.ct, 0x7ff00000u);
+    ok &= rn_ordinary(r.ct);
     if (!ok) r = multipole_steps_call<BEND, false>(in, e, pm, nl1, nl2);
 }
 

@@ -379,8 +379,8 @@ __device__ __forceinline__ void multipole_steps_generic(P6T<T>* r, const Rec& e,
 
 /* The Forest-Ruth steps of a thick multipole by the reference's plain
  * expressions (StrMPoleSymplectic4Pass.c:73-93 and the Bnd and Rad variants);
- * pn0: 1/(1+delta) of the element's entry, which scales the drift lengths of
- * the non-radiating variants. */
+ * nl1, nl2: the drift lengths of the non-radiating variants, scaled by
+ * 1/(1+delta) of the element's entry. */
 template <int NP, bool BEND, bool RAD, class PL, class T>
 __device__ __forceinline__ void multipole_steps_plain(P6T<T>* r, const Rec& e, const PL& pl,
                                                       const T* nl1, const T* nl2, double irho,
@@ -444,16 +444,22 @@ __device__ __noinline__ P6 multipole_steps_call(P6 r, Rec e, Param pm, double nl
  * The divisions bounded these loops: about nine FP64 instructions each, a
  * seed on the XU pipe and a branch to a slow path that ended the block the
  * compiler could interleave (a plain sextupole step of a lone warp took 631
- * cycles and takes 275, a radiating one 1886 and 946; of 16 warps a scheduler
- * each takes 296 and now 160 cycles a plain step, 836 and 498 a radiating
- * one).  The last drift of a step and the
- * first of the next have the same length, momenta and 1/(1+delta), hence the
- * same increments: they are computed once and added twice.  A warp with an
- * operand out of range pays for both loops, which only particles about to be
- * lost do.  Returns 1/(1+delta) at the exit of a radiating magnet. */
+ * cycles and takes 275, of 16 warps a scheduler 296 and 160).  The last drift
+ * of a step and the first of the next have the same length, momenta and
+ * 1/(1+delta), hence the same increments: they are computed once and added
+ * twice.
+ * Conditions belong outside the loop, where they do not wait for the kicks:
+ * with the path factor, the angles and the roundings next to one tested in
+ * every kick a turn of the large ring took 5.2 ms for one warp an SM and 40.9
+ * for 300,000 particles, with the largest loss alone kept there and the rest
+ * at the ends 4.35 and 34.5.  Out of range are energy losses above 2^-14 in
+ * one kick of a bend (2^-18 with more than 256 steps), 2^-18 in a straight
+ * magnet, 1 + delta outside [97/128, 5/4) ([1/2, 2) without radiation), and
+ * what overflows: particles about to be lost.  Such a magnet is tracked again
+ * from its entry; one that is out of range there takes a single step first. */
 template <int NP, bool BEND, bool RAD, class PL>
 __device__ __forceinline__ void multipole_steps_rn(P6* r, Recip* c, const Rec& e, const PL& pl,
-                                                   const Param& pm, const double* dp0,
+                                                   const Param& pm, const double* pb,
                                                    const double* nl1, const double* nl2,
                                                    double irho, int ns) {
     if (ns <= 0) return;
@@ -465,34 +471,42 @@ __device__ __forceinline__ void multipole_steps_rn(P6* r, Recip* c, const Rec& e
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         in[k] = r[k];
-        ok[k] = (e.flags() & ATB_F_RN) && rn_opd_fits(1.0 + r[k].dp) &&
-                rn_coords_fit(r[k].x, r[k].px, r[k].y, r[k].py);
+        ok[k] = (e.flags() & ATB_F_RN) &&
+                (RAD ? rn_opd_fits(1.0 + r[k].dp) &&
+                           rn_coords_fit(r[k].x, r[k].px, r[k].y, r[k].py)
+                     : rn_opd_constant(1.0 + r[k].dp));
     }
+    /* out of range already: a single step here, for nothing */
+    int m = ns;
+#pragma unroll
+    for (int k = 0; k < NP; ++k)
+        if (ok[k]) m = 1;
     if (RAD) {
         const double L1 = e.f(ATB_SM_L1), L2 = e.f(ATB_SM_L2), radc = e.f(ATB_SM_RADC);
         double o[NP], pn[NP];
+        uint32_t loss[NP];             /* the largest kick's, its high word */
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
             o[k] = 1.0 + r[k].dp;
             pn[k] = opd_rcp(c[k], r[k].dp);
-            ok[k] &= !rn_denormal(r[k].px) && !rn_denormal(r[k].py);
+            loss[k] = 0u;
             d1[k] = drift_rad_inc(r[k], L1, pn[k]);
             add_drift_rad(r[k], d1[k]);
         }
-        for (int m = 1;; ++m) {
+        for (;; ++m) {
 #pragma unroll
             for (int k = 0; k < NP; ++k)
-                kick_rad_rn<BEND>(r[k], pl, K1, irho, k1i, radc, o[k], pn[k], ok[k]);
+                kick_rad_rn<BEND>(r[k], pl, K1, irho, k1i, radc, o[k], pn[k], loss[k]);
 #pragma unroll
             for (int k = 0; k < NP; ++k) add_drift_rad(r[k], drift_rad_inc(r[k], L2, pn[k]));
 #pragma unroll
             for (int k = 0; k < NP; ++k)
-                kick_rad_rn<BEND>(r[k], pl, K2, irho, k2i, radc, o[k], pn[k], ok[k]);
+                kick_rad_rn<BEND>(r[k], pl, K2, irho, k2i, radc, o[k], pn[k], loss[k]);
 #pragma unroll
             for (int k = 0; k < NP; ++k) add_drift_rad(r[k], drift_rad_inc(r[k], L2, pn[k]));
 #pragma unroll
             for (int k = 0; k < NP; ++k)
-                kick_rad_rn<BEND>(r[k], pl, K1, irho, k1i, radc, o[k], pn[k], ok[k]);
+                kick_rad_rn<BEND>(r[k], pl, K1, irho, k1i, radc, o[k], pn[k], loss[k]);
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 d1[k] = drift_rad_inc(r[k], L1, pn[k]);
@@ -504,7 +518,9 @@ __device__ __forceinline__ void multipole_steps_rn(P6* r, Recip* c, const Rec& e
         }
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
-            ok[k] &= rn_not_tiny(r[k].px) && rn_not_tiny(r[k].py);
+            ok[k] &= loss[k] < (BEND ? rn_seed_wide_hi(ns) : ATB_RN_SEED_HI) &&
+                     rn_ordinary(r[k].x) && rn_ordinary(r[k].px) && rn_ordinary(r[k].y) &&
+                     rn_ordinary(r[k].py);
             c[k].dp = r[k].dp;
             c[k].pn = pn[k];
         }
@@ -512,46 +528,43 @@ __device__ __forceinline__ void multipole_steps_rn(P6* r, Recip* c, const Rec& e
         double od2[NP], hp[NP];
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
-            const double o = 1.0 + r[k].dp;
-            od2[k] = 2.0 * o;
-            hp[k] = 0.5 * c[k].pn;
-            /* the cached reciprocal is the entry's: an entrance shift may
-               have changed delta since */
-            ok[k] &= r[k].dp == dp0[k];
-            d1[k] = fastdrift_inc(r[k], nl1[k], od2[k], hp[k], ok[k]);
+            od2[k] = 2.0 * (1.0 + r[k].dp);
+            hp[k] = 0.5 * pb[k];
+            d1[k] = fastdrift_inc(r[k], nl1[k], od2[k], hp[k]);
             add_drift(r[k], d1[k]);
         }
-        for (int m = 1;; ++m) {
+        for (;; ++m) {
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
             }
 #pragma unroll
             for (int k = 0; k < NP; ++k)
-                add_drift(r[k], fastdrift_inc(r[k], nl2[k], od2[k], hp[k], ok[k]));
+                add_drift(r[k], fastdrift_inc(r[k], nl2[k], od2[k], hp[k]));
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 if (BEND) bndthinkick(r[k], pl, K2, irho, k2i); else strthinkick(r[k], pl, K2);
             }
 #pragma unroll
             for (int k = 0; k < NP; ++k)
-                add_drift(r[k], fastdrift_inc(r[k], nl2[k], od2[k], hp[k], ok[k]));
+                add_drift(r[k], fastdrift_inc(r[k], nl2[k], od2[k], hp[k]));
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 if (BEND) bndthinkick(r[k], pl, K1, irho, k1i); else strthinkick(r[k], pl, K1);
             }
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
-                d1[k] = fastdrift_inc(r[k], nl1[k], od2[k], hp[k], ok[k]);
+                d1[k] = fastdrift_inc(r[k], nl1[k], od2[k], hp[k]);
                 add_drift(r[k], d1[k]);
             }
             if (m == ns) break;
 #pragma unroll
             for (int k = 0; k < NP; ++k) add_drift(r[k], d1[k]);
         }
-        /* an overflow anywhere has reached ct */
+        /* an overflow anywhere has reached ct; it is also where the
+           quotients have gone */
 #pragma unroll
-        for (int k = 0; k < NP; ++k) ok[k] &= rn_below(r[k].ct, 0x7ff00000u);
+        for (int k = 0; k < NP; ++k) ok[k] &= rn_ordinary(r[k].ct);
     }
 #pragma unroll
     for (int k = 0; k < NP; ++k)
@@ -657,7 +670,7 @@ __device__ __forceinline__ void multipole_steps_fast(P6* r, Recip* c, const Rec&
  * (-1: read from the table on every kick). */
 template <int NP, int MO, bool BEND, bool RAD, bool SKEW>
 __device__ __forceinline__ void multipole_steps_mo(P6* r, Recip* c, const Rec& e, const Param& pm,
-                                                   const double* dp0, const double* nl1,
+                                                   const double* pb, const double* nl1,
                                                    const double* nl2, double irho, int ns) {
     const int mo = e.mo();
     const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
@@ -665,12 +678,12 @@ __device__ __forceinline__ void multipole_steps_mo(P6* r, Recip* c, const Rec& e
     pl.load(A, A + mo + 1, mo);
     if (pm.k >= 0) pl.set_param(pm.k, pm.v);
     if constexpr (kFast) multipole_steps_fast<NP, BEND, RAD>(r, c, e, pl, nl1, nl2, irho, ns);
-    else multipole_steps_rn<NP, BEND, RAD>(r, c, e, pl, pm, dp0, nl1, nl2, irho, ns);
+    else multipole_steps_rn<NP, BEND, RAD>(r, c, e, pl, pm, pb, nl1, nl2, irho, ns);
 }
 
 template <int NP, bool BEND, bool RAD, bool INTEG, class T>
 __device__ __forceinline__ void multipole_steps(P6T<T>* r, RecipOf<T>* c, const Rec& e,
-                                                const Param& pm, const double* dp0, const T* nl1,
+                                                const Param& pm, const double* pb, const T* nl1,
                                                 const T* nl2, double irho, int ns) {
     if constexpr (is_dual<T>::value) {
         /* one generic instance for the tangent kernel keeps its size sane */
@@ -691,7 +704,7 @@ __device__ __forceinline__ void multipole_steps(P6T<T>* r, RecipOf<T>* c, const 
         multipole_steps_generic<NP, BEND, RAD>(r, e, pl, nl2, irho, ns);
     } else {
 #define ATB_STEPS(MO, SKEW) \
-    multipole_steps_mo<NP, MO, BEND, RAD, SKEW>(r, c, e, pm, dp0, nl1, nl2, irho, ns)
+    multipole_steps_mo<NP, MO, BEND, RAD, SKEW>(r, c, e, pm, pb, nl1, nl2, irho, ns)
         /* upright magnets' fields without the zero skew terms */
         const bool upright = e.flags() & ATB_F_NOSKEW;
         switch (e.mo()) {
@@ -729,21 +742,25 @@ template <int NP, bool BEND, bool RAD, bool INTEG = false, bool LEAN = false, cl
 __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const Rec& e,
                                                  const Param& pm) {
     const uint32_t fl = e.flags();
-    double dp0[NP];
+    double pb[NP];             /* 1/(1+delta) in the body of a plain magnet */
     T nl1[NP], nl2[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         if (!LEAN && (fl & ATB_F_SCALING)) change_pref<kFast>(r[k], e.f(ATB_SM_SCALE));
-        dp0[k] = val(r[k].dp);
+        pb[k] = 0.0;
         nl1[k] = 0.0;
         nl2[k] = 0.0;
         if (!RAD) {
             T p_norm = opd_rcp(c[k], r[k].dp);
+            pb[k] = val(p_norm);
             nl1[k] = e.f(ATB_SM_L1) * p_norm;
             nl2[k] = e.f(ATB_SM_L2) * p_norm;
         }
         if (e.opt) {
+            const double dp0 = val(r[k].dp);
             entrance_misalign<LEAN>(r[k], e);
+            /* a shift or a dense rotation may change delta */
+            if (!RAD && val(r[k].dp) != dp0) pb[k] = 1.0 / (1.0 + val(r[k].dp));
             apertures<LEAN>(r[k], e);
         }
     }
@@ -777,7 +794,7 @@ __device__ __forceinline__ void pass_multipole_n(P6T<T>* r, RecipOf<T>* c, const
             }
         }
     }
-    multipole_steps<NP, BEND, RAD, INTEG>(r, c, e, pm, dp0, nl1, nl2, irho, e.nsteps());
+    multipole_steps<NP, BEND, RAD, INTEG>(r, c, e, pm, pb, nl1, nl2, irho, e.nsteps());
     if (!LEAN && (fl & ATB_F_FQ_OUT)) {
         const T b1 = fringe_b1<T>(e, pm);
 #pragma unroll

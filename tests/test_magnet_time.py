@@ -32,6 +32,7 @@ def _bend(length=0.05, rho=7.0):
 
 #: name: (element, energy in eV, coordinate, its size at the reference, its size outside)
 CASES = {
+    "off momentum, no radiation": (E.Quadrupole("Q", 0.2, 1e-3), 3e9, 4, 1e-4, 3e-1),
     "angles": (_quad(), 3e9, 1, 1e-4, 3e-2),
     "far from a bend's axis": (_bend(), 3e9, 0, 1e-5, 4e-2),
     "a compact bend": (_bend(rho=1.0), 1e9, 0, 1e-5, 2e-2),
@@ -64,16 +65,27 @@ def _time(el, energy, coord, size, mode):
     return best
 
 
-@pytest.mark.parametrize("mode", ["fast"])
+@pytest.mark.parametrize("mode", ["exact", "fast"])
 @pytest.mark.parametrize("case", sorted(CASES))
 def test_time_does_not_depend_on_the_coordinates(case, mode):
     el, energy, coord, near, far = CASES[case]
     assert _time(el, energy, coord, far, mode) <= 1.25 * _time(el, energy, coord, near, mode)
 
 
-@pytest.mark.parametrize("mode", ["fast"])
+@pytest.mark.parametrize("mode", ["exact", "fast"])
 @pytest.mark.parametrize("energy", sorted(DIPOLES))
 def test_time_does_not_depend_on_the_energy_loss(energy, mode):
     length, angle = DIPOLES[energy]
     el = E.Dipole("B", length, angle, PassMethod=RAD % "Bnd")
     assert _time(el, energy, 0, 1e-5, mode) <= 1.25 * _time(el, 1e9, 0, 1e-5, mode)
+
+
+@pytest.mark.parametrize("mode", ["exact", "fast"])
+def test_time_does_not_depend_on_what_an_entrance_rotation_mixes(mode):
+    """A dense rotation that changes delta takes a division more a magnet than
+    one that leaves it."""
+    keep = np.eye(6) + 1e-9 * np.random.default_rng(0).standard_normal((6, 6))
+    mixes = keep.copy()
+    keep[4] = np.eye(6)[4]
+    times = [_time(E.Quadrupole("Q", 0.2, 1e-3, R1=r), 3e9, 0, 1e-6, mode) for r in (mixes, keep)]
+    assert times[0] <= 1.25 * times[1]
