@@ -135,15 +135,22 @@ struct Rec {
 /* ---------------- misalignment / aperture wrappers ----------------------- */
 
 #define ATB_OPT_FIELD(slot) ((uint64_t)ATB_OPT_MASK << ((slot) * ATB_OPT_BITS))
+#define ATB_OPT_APERTURES (ATB_OPT_FIELD(ATB_OPT_RAP) | ATB_OPT_FIELD(ATB_OPT_EAP))
 
 static __device__ __noinline__ P6 mult_dense_call(P6 r, const double* m) {
     mult_dense(r, m);
     return r;
 }
-static __device__ __noinline__ double apertures_call(P6 r, Rec e) {
-    if (const double* ra = e.blk(ATB_OPT_RAP)) check_rect(r, ra);
-    if (const double* ea = e.blk(ATB_OPT_EAP)) check_ellip(r, ea);
-    return r.ct;
+/* whether (x, y) is outside an element's apertures (null: none) */
+static __device__ __noinline__ bool outside_call(double x, double y, const double* rect,
+                                                 const double* ellip) {
+    P6 r;
+    r.x = x;
+    r.y = y;
+    r.ct = 0.0;
+    if (rect) check_rect(r, rect);
+    if (ellip) check_ellip(r, ellip);
+    return r.ct != 0.0;
 }
 
 /* CALL: the rare forms out of line */
@@ -206,8 +213,8 @@ __device__ __forceinline__ void entrance_misalign(P6T<T>& r, const Rec& e) {
 template <bool CALL = false, class T>
 __device__ __forceinline__ void apertures(P6T<T>& r, const Rec& e) {
     if constexpr (CALL) {
-        if (e.opt & (ATB_OPT_FIELD(ATB_OPT_RAP) | ATB_OPT_FIELD(ATB_OPT_EAP)))
-            r.ct = apertures_call(r, e);
+        if (__builtin_expect((e.opt & ATB_OPT_APERTURES) != 0, 0))
+            if (outside_call(r.x, r.y, e.blk(ATB_OPT_RAP), e.blk(ATB_OPT_EAP))) r.ct = inf_d();
     } else {
         if (const double* ra = e.blk(ATB_OPT_RAP)) check_rect(r, ra);
         if (const double* ea = e.blk(ATB_OPT_EAP)) check_ellip(r, ea);
@@ -705,23 +712,24 @@ __device__ __forceinline__ void multipole_steps(P6T<T>* r, RecipOf<T>* c, const 
     } else {
 #define ATB_STEPS(MO, SKEW) \
     multipole_steps_mo<NP, MO, BEND, RAD, SKEW>(r, c, e, pm, pb, nl1, nl2, irho, ns)
-        /* upright magnets' fields without the zero skew terms */
+        /* upright magnets' fields without the zero skew terms; the loops that
+           most magnets run first, for the compiler to lay them side by side */
         const bool upright = e.flags() & ATB_F_NOSKEW;
-        switch (e.mo()) {
-            case 0: ATB_STEPS(0, true); break;
-            case 1:
-                if (upright) ATB_STEPS(1, false);
-                else ATB_STEPS(1, true);
-                break;
-            case 2:
-                if (upright) ATB_STEPS(2, false);
-                else ATB_STEPS(2, true);
-                break;
-            case 3:
-                if (upright) ATB_STEPS(3, false);
-                else ATB_STEPS(3, true);
-                break;
-            default: ATB_STEPS(-1, true); break;
+        const int mo = e.mo();
+        if (__builtin_expect(upright && mo == 1, 1)) {
+            ATB_STEPS(1, false);
+        } else if (__builtin_expect(upright && mo == 2, 1)) {
+            ATB_STEPS(2, false);
+        } else if (__builtin_expect(upright && mo == 3, 1)) {
+            ATB_STEPS(3, false);
+        } else {
+            switch (mo) {
+                case 0: ATB_STEPS(0, true); break;
+                case 1: ATB_STEPS(1, true); break;
+                case 2: ATB_STEPS(2, true); break;
+                case 3: ATB_STEPS(3, true); break;
+                default: ATB_STEPS(-1, true); break;
+            }
         }
 #undef ATB_STEPS
     }
@@ -966,6 +974,17 @@ static __device__ __noinline__ P6 track_element_call(P6 r, Rec e, int nturn, Par
     return r;
 }
 
+/* the field of a thin multipole, out of line: only x and y go there */
+static __device__ __noinline__ double2 field_call(double x, double y, const double* A, int mo,
+                                                  Param pm) {
+    Poly<-1> pl;
+    pl.load(A, A + mo + 1, mo);
+    if (pm.k >= 0) pl.set_param(pm.k, pm.v);
+    double2 f;
+    pl.field(x, y, f.x, f.y);
+    return f;
+}
+
 /* A magnet of a table compiled for another integrator of the GPU call, in the
  * kernels built with them (GEN); the hosts of the other kernels send them none
  * (atb_track_noalloc checks its raw table with a scan kernel, the tangent host
@@ -981,11 +1000,15 @@ __device__ __forceinline__ void track_integ(P6& r, Recip& c, const Rec& e, const
 
 /* One element on one particle; lost particles (x is NaN) are skipped as every
  * reference pass method does (e.g. StrMPoleSymplectic4Pass.c:59).  Only what
- * most of a lattice consists of is in line (CALL: drifts only): with cavities, correctors, thin
- * multipoles, fringes and the rest beside them the particle moved between
- * registers around every element (159 instructions for a drift, 14 of them
- * FP64, where it now takes 88; a quadrupole beside its steps 1,060 cycles of a
- * lone warp instead of 1,400). */
+ * most of a lattice consists of is in line: drifts, magnets (not with CALL),
+ * markers, plain correctors, and of thin multipoles and apertures all but the
+ * arithmetic on x and y.  With cavities, fringes and the rest beside them the
+ * particle moved between registers around every element (159 instructions for
+ * a drift, 14 of them FP64, where it now takes 88; a quadrupole beside its
+ * steps 1,060 cycles of a lone warp instead of 1,400).  A call that takes and
+ * returns the whole particle costs some 600 cycles: with it a marker took 1,400,
+ * now 720, a thin multipole 2,000, now 1,200, a drift with apertures 2,300, now
+ * 1,700. */
 template <bool GEN = false, bool CALL = false, class T>
 __device__ __forceinline__ void track_element(P6T<T>& r, RecipOf<T>& c, const Rec& e, int nturn,
                                               const Param& pm = Param{-1, 0.0},
@@ -1025,6 +1048,30 @@ __device__ __forceinline__ void track_element(P6T<T>& r, RecipOf<T>& c, const Re
                 pass_multipole_n<1, true, true, false, true>(&r, &c, e, pm);
                 return;
             }
+        }
+        if (op == ATB_OP_IDENTITY && e.opt == 0) return;
+        if (op == ATB_OP_CORRECTOR && e.opt == 0 &&
+            !(e.flags() & (ATB_F_SCALING | ATB_F_THICK))) {
+            r.px += e.f(ATB_CO_XK);
+            r.py += e.f(ATB_CO_YK);
+            return;
+        }
+        if (__builtin_expect(op == ATB_OP_DRIFT && !(e.opt & ~ATB_OPT_APERTURES), 0)) {
+            apertures<true>(r, e);
+            drift6_pn<kFast>(r, e.f(ATB_DR_LE), opd_rcp(c, r.dp));
+            apertures<true>(r, e);
+            return;
+        }
+        if (__builtin_expect(op == ATB_OP_THINMPOLE && e.opt == 0 &&
+                             !(e.flags() & ATB_F_SCALING), 0)) {
+            const double2 f = field_call(r.x, r.y, e.p + ATB_TM_POLY, e.mo(), pm);
+            const double bax = e.f(ATB_TM_BAX), bay = e.f(ATB_TM_BAY);
+            r.px = msub(r.px, 1.0, f.x);
+            r.py = madd(r.py, 1.0, f.y);
+            r.px += bax * r.dp;
+            r.py -= bay * r.dp;
+            r.ct -= bax * r.x - bay * r.y;
+            return;
         }
         r = track_element_call(r, e, nturn, pm, rng, p, ei);
     }
