@@ -19,21 +19,23 @@
  * forward pass stored every turn's (memory permitting); then
  * atb_adjoint_turn_kernel walks the elements backwards with
  * lambda <- J_e^T lambda, J_e the element's Jacobian at its stored entry
- * state, and at an element that carries K_q, dL/dK_q += (d r_out / d K_q) . lambda_out, summed over the
- * block's particles in shared memory and added to the global sum once per
- * block.
+ * state, and at an element that carries K_q,
+ * dL/dK_q += (d r_out / d K_q) . lambda_out, summed over the block's particles
+ * in shared memory and added to the global sum once per block.
  *
  * Element adjoints:
  *  - DriftPass, IdentityPass, AperturePass, RFCavityPass, thin
  *    CorrectorPass, ThinMPolePass and the non-radiating StrMPole/BndMPole
  *    Symplectic4 passes (plain or bend-edge entrance/exit, misaligned or
- *    not): written out by hand.  A thick magnet is walked
- *    backwards from its exit state (the next element's entry state): every
- *    stage is undone on (x, px, y, py) -- a drift or kick is its own inverse
- *    but for the sign -- and reversed at the coordinates so found: the
- *    fastdrift (driftkick.c:37-48), and the kick (driftkick.c:51-115) with the
- *    field derivative F'(z) of F(z) = sum (B_n + i A_n) z^n from a second
- *    Horner recursion and dF/dB_k = z^k for the strength.
+ *    not): written out by hand.  A thick magnet is walked backwards from its
+ *    exit state (the next element's entry state): every stage is undone on
+ *    (x, px, y, py) -- a drift or kick is its own inverse but for the sign --
+ *    and reversed at the coordinates so found: the fastdrift
+ *    (driftkick.c:37-48), and the kick (driftkick.c:51-115) with the field
+ *    derivative F'(z) of F(z) = sum (B_n + i A_n) z^n from a second Horner
+ *    recursion and dF/dB_k = z^k for the strength.  In a magnet of a focusing
+ *    phase above two radians, where the undone coordinates would lose digits,
+ *    the steps' entry states are kept instead (adj_strong_magnet).
  *  - every other element (radiating magnets, quadrupole fringes, field
  *    scaling, thick correctors, bend edges of method 3): J_e from a
  *    forward-mode evaluation of the whole element on dual numbers (6
@@ -409,12 +411,110 @@ __device__ __forceinline__ bool adj_by_hand(const Rec& e, bool bend) {
     return true;
 }
 
+/* Undoing a stage rounds its coordinates, and the roundings grow by the inverse
+ * of the magnet's map as the walk goes on: relative to the coordinates by about
+ * exp(2 phi), phi^2 = |F'| L^2 the magnet's (worst) focusing phase.  Up to phi
+ * = 2 dL/d r is as close to the tangent's as with forward coordinates (2e-15 of
+ * its terms); the delta column is off by 6e-15 at phi = 3 and 2e-12 at 6.
+ * Quadrupoles of the FODO and large ring have 0.5 and 0.6.  Stronger magnets,
+ * at this particle's ends of it, keep their step entries (adj_strong_magnet).
+ * k, nl: the magnet's kick and drift lengths. */
+template <class C>
+__device__ __forceinline__ bool adj_strong(const C& c, const XY& in, const XY& out, double k,
+                                           double nl, double irho) {
+    double ar, ai, br, bi;
+    c.prime(in.x, in.y, ar, ai);
+    c.prime(out.x, out.y, br, bi);
+    const double f = fmax(fabs(ar) + fabs(ai), fabs(br) + fabs(bi));
+    return fma(irho, irho, f) * fabs(k * nl) > 4.0;
+}
+
+/* A magnet in reverse with every coordinate found forwards: the transverse
+ * coordinates entering its steps are kept (all of up to ten, every
+ * ceil(n / 10)-th of more, the others tracked again from the nearest), each
+ * step is run again with the inputs of its stages kept, and the stages are
+ * reversed.  Twice the work of undoing them. */
+template <bool BEND>
+__device__ __noinline__ Lam6 adj_strong_magnet(P6 s, Lam6 io, Rec e, Param pm) {
+    constexpr int KEEP = 10;
+    double* lam = io.v;
+    const uint32_t fl = e.flags();
+    const double K1 = e.f(ATB_SM_K1), K2 = e.f(ATB_SM_K2);
+    const int mo = e.mo(), ns = e.nsteps();
+    const double* A = e.p + (BEND ? ATB_BM_POLY : ATB_SM_POLY);
+    AdjCoef<-1, true> c;
+    c.load(A, A + mo + 1, mo, pm.k, pm.v);
+    const double pn0 = 1.0 / (1.0 + s.dp);
+    const double nl1 = e.f(ATB_SM_L1) * pn0, nl2 = e.f(ATB_SM_L2) * pn0;
+    const double irho = BEND ? e.f(ATB_BM_IRHO) : 0.0;
+    const double k1i = BEND ? e.f(ATB_BM_K1IRHO) : 0.0, k2i = BEND ? e.f(ATB_BM_K2IRHO) : 0.0;
+    const int m_in = (int)((fl >> ATB_F_BM_IN_SHIFT) & ATB_F_BM_MASK);
+    const int m_out = (int)((fl >> ATB_F_BM_OUT_SHIFT) & ATB_F_BM_MASK);
+    P6 r = s;
+    entrance_misalign(r, e);
+    const double dp = r.dp;
+    XY q{r.x, r.px, r.y, r.py};
+    if (BEND) {
+        q.px = fma(q.x, e.f(ATB_BM_FXIN), q.px);
+        q.py = fma(-q.y, adj_edge_fy(dp, irho, e, ATB_BM_EIN, m_in, fl & ATB_F_FC0_IN), q.py);
+    }
+    auto step = [&](XY& t) {
+        xy_drift(t, nl1);
+        xy_kick<BEND>(t, c, K1, irho, dp);
+        xy_drift(t, nl2);
+        xy_kick<BEND>(t, c, K2, irho, dp);
+        xy_drift(t, nl2);
+        xy_kick<BEND>(t, c, K1, irho, dp);
+        xy_drift(t, nl1);
+    };
+    XY keep[KEEP];
+    const int stride = ns > KEEP ? (ns + KEEP - 1) / KEEP : 1;
+    for (int m = 0; m < ns; ++m) {
+        if (m % stride == 0) keep[m / stride] = q;
+        step(q);
+    }
+    adj_exit_misalign(lam, e);
+    const double h = 0.5 / (1.0 + dp), lc = lam[5], cc = 2.0 * h * lc;
+    const double c1 = cc * nl1, c2 = cc * nl2;
+    if (BEND) adj_edge(q.y, dp, lam, irho, e, ATB_BM_EOUT, m_out, fl & ATB_F_FC0_OUT);
+    DriftSums d1{0.0, 0.0}, d2{0.0, 0.0};
+    for (int m = ns - 1; m >= 0; --m) {
+        XY t = keep[m / stride];
+        for (int j = (m / stride) * stride; j < m; ++j) step(t);
+        const XY t0 = t;
+        xy_drift(t, nl1);
+        const XY t1 = t;
+        xy_kick<BEND>(t, c, K1, irho, dp);
+        xy_drift(t, nl2);
+        const XY t3 = t;
+        xy_kick<BEND>(t, c, K2, irho, dp);
+        xy_drift(t, nl2);
+        const XY t5 = t;
+        xy_kick<BEND>(t, c, K1, irho, dp);
+        adj_fastdrift(t.px, t.py, nl1, c1, lam, d1);
+        adj_kick<BEND>(c, t5.x, t5.y, K1, k1i, irho, lam, io.g);
+        adj_fastdrift(t5.px, t5.py, nl2, c2, lam, d2);
+        adj_kick<BEND>(c, t3.x, t3.y, K2, k2i, irho, lam, io.g);
+        adj_fastdrift(t3.px, t3.py, nl2, c2, lam, d2);
+        adj_kick<BEND>(c, t1.x, t1.y, K1, k1i, irho, lam, io.g);
+        adj_fastdrift(t0.px, t0.py, nl1, c1, lam, d1);
+    }
+    double lnl = 0.0;
+    adj_drift_sums(d1, nl1, h, lc, lam, lnl);
+    adj_drift_sums(d2, nl2, h, lc, lam, lnl);
+    if (BEND) adj_edge(r.y, dp, lam, irho, e, ATB_BM_EIN, m_in, fl & ATB_F_FC0_IN);
+    adj_entrance_misalign(lam, e);
+    lam[4] = fma(-lnl, pn0, lam[4]);
+    return io;
+}
+
 /* StrMPoleSymplectic4Pass.c:29-109 / BndMPoleSymplectic4Pass.c:38-129 in
  * reverse, from the entry state s and the exit state sx.  A magnet with
  * misalignments or apertures of its own finds the body's exit by tracking the
- * body again (undoing a rotation would need its inverse). */
+ * body again (undoing a rotation would need its inverse).  False: the magnet is
+ * a strong one, nothing done. */
 template <bool BEND, int MO, bool SKEW, bool PLAIN = false>
-__device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Recip& rc,
+__device__ __forceinline__ bool adj_multipole_mo(const P6& s, const P6& sx, Recip& rc,
                                                  double* lam, const Rec& e, const Param& pm,
                                                  double& g) {
     const uint32_t fl = e.flags();
@@ -431,13 +531,13 @@ __device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Reci
     const int m_out = (int)((fl >> ATB_F_BM_OUT_SHIFT) & ATB_F_BM_MASK);
 
     /* q: leaving the body, before the exit edge */
-    XY q{sx.x, sx.px, sx.y, sx.py};
+    XY q{sx.x, sx.px, sx.y, sx.py}, q0{s.x, s.px, s.y, s.py};
     double dp = sx.dp;                       /* constant through the magnet */
     if (!PLAIN && e.opt) {
         P6 r = s;
         entrance_misalign(r, e);
         dp = r.dp;
-        q = XY{r.x, r.px, r.y, r.py};
+        q = q0 = XY{r.x, r.px, r.y, r.py};
         if (BEND) {
             q.px = fma(q.x, e.f(ATB_BM_FXIN), q.px);
             q.py = fma(-q.y, adj_edge_fy(dp, irho, e, ATB_BM_EIN, m_in, fl & ATB_F_FC0_IN), q.py);
@@ -449,6 +549,9 @@ __device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Reci
             xy_kick<BEND>(q, c, mid ? K2 : K1, irho, dp);
         }
         if (ns > 0) xy_drift(q, nl1);
+    }
+    if (adj_strong(c, q0, q, fma(2.0, K1, K2) * ns, 2.0 * (nl1 + nl2) * ns, irho)) return false;
+    if (!PLAIN && e.opt) {
         adj_exit_misalign(lam, e);
     } else if (BEND) {
         q.px = fma(-q.x, e.f(ATB_BM_FXOUT), q.px);
@@ -489,6 +592,7 @@ __device__ __forceinline__ void adj_multipole_mo(const P6& s, const P6& sx, Reci
     if (!PLAIN && e.opt) adj_entrance_misalign(lam, e);
     /* nl = L / (1 + dp) of the entry momentum */
     lam[4] = fma(-lnl, pn0, lam[4]);
+    return true;
 }
 
 template <bool BEND>
@@ -497,11 +601,21 @@ __device__ __forceinline__ void adj_pass_multipole(const P6& s, const P6& sx, Re
                                                    double& g) {
     const bool upright = e.flags() & ATB_F_NOSKEW;
     const int mo = e.mo();
-    if (mo == 1 && upright) adj_multipole_mo<BEND, 1, false>(s, sx, rc, lam, e, pm, g);
-    else if (mo == 2 && upright) adj_multipole_mo<BEND, 2, false>(s, sx, rc, lam, e, pm, g);
-    else if (mo == 3 && upright) adj_multipole_mo<BEND, 3, false>(s, sx, rc, lam, e, pm, g);
-    else if (mo == 0) adj_multipole_mo<BEND, 0, true>(s, sx, rc, lam, e, pm, g);
-    else adj_multipole_mo<BEND, -1, true>(s, sx, rc, lam, e, pm, g);
+    bool done;
+    if (mo == 1 && upright) done = adj_multipole_mo<BEND, 1, false>(s, sx, rc, lam, e, pm, g);
+    else if (mo == 2 && upright) done = adj_multipole_mo<BEND, 2, false>(s, sx, rc, lam, e, pm, g);
+    else if (mo == 3 && upright) done = adj_multipole_mo<BEND, 3, false>(s, sx, rc, lam, e, pm, g);
+    else if (mo == 0) done = adj_multipole_mo<BEND, 0, true>(s, sx, rc, lam, e, pm, g);
+    else done = adj_multipole_mo<BEND, -1, true>(s, sx, rc, lam, e, pm, g);
+    if (done) return;
+    Lam6 io;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) io.v[i] = lam[i];
+    io.g = g;
+    io = adj_strong_magnet<BEND>(s, io, e, pm);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) lam[i] = io.v[i];
+    g = io.g;
 }
 
 /* ---- thin elements -------------------------------------------------------- */
@@ -651,12 +765,11 @@ __device__ __forceinline__ void adj_element(const P6& s, const P6& sx, Recip& rc
         return;
     }
     if (op == ATB_OP_STRMPOLE && plain && upright && adj_by_hand(e, false)) {
-        if (mo == 1) { adj_multipole_mo<false, 1, false, true>(s, sx, rc, lam, e, pm, g); return; }
-        if (mo == 2) { adj_multipole_mo<false, 2, false, true>(s, sx, rc, lam, e, pm, g); return; }
+        if (mo == 1 && adj_multipole_mo<false, 1, false, true>(s, sx, rc, lam, e, pm, g)) return;
+        if (mo == 2 && adj_multipole_mo<false, 2, false, true>(s, sx, rc, lam, e, pm, g)) return;
     }
     if (op == ATB_OP_BNDMPOLE && plain && upright && mo == 1 && adj_by_hand(e, true)) {
-        adj_multipole_mo<true, 1, false, true>(s, sx, rc, lam, e, pm, g);
-        return;
+        if (adj_multipole_mo<true, 1, false, true>(s, sx, rc, lam, e, pm, g)) return;
     }
     Lam6 io;
 #pragma unroll
