@@ -1,7 +1,7 @@
 /*
  * The tangent kernel of lattices whose elements all have a hand-written
- * derivative (tangent_by_hand below): drifts, non-radiating magnets, thin
- * multipoles and correctors, cavities, apertures.
+ * derivative (atb_tangent_by_hand of atb_table.h): drifts, non-radiating
+ * magnets, thin multipoles and correctors, cavities, apertures.
  *
  * The general tangent kernel runs every operation on dual numbers of seven
  * slots.  Here a magnet's steps carry the particle (by the exact kernels' own
@@ -28,7 +28,6 @@
 
 namespace atb {
 
-
 /* The particle's tangent map in shared memory, entry (i, j) at
  * base[(6 i + j) * ATB_TANGENT_THREADS]: a warp's accesses are consecutive. */
 struct TanMap {
@@ -46,10 +45,23 @@ struct TanCol {
 
 /* The columns: with respect to x, px, y, py, delta (c[0..4]) and to the
  * differentiated strength (c[5]).  In a decoupled magnet (DEC) the x columns
- * have no y entries and the y columns no x entries. */
+ * have no y entries and the y columns no x entries.  They hold what the magnet
+ * adds to a drift as long as the stages so far: to 1 in dx/dx, dpx/dpx, dy/dy,
+ * dpy/dpy, to the length s (over 1 + delta) in dx/dpx and dy/dpy, to sx and sy
+ * in dct/dpx and dct/dpy.  Equal magnets round alike, so that the errors of
+ * their Jacobians add up over a ring; with whole entries, rounded at the size
+ * of one in every stage, the dispersion and ct terms of the FODO ring were off
+ * by 1.4 times what the dual numbers leave. */
 struct TanCols {
     TanCol c[6];
+    double s, sx, sy;
 };
+__device__ __forceinline__ double tan_x(const TanCols& t, int j) {
+    return j == 0 ? 1.0 + t.c[0].x : j == 1 ? t.s + t.c[1].x : t.c[j].x;
+}
+__device__ __forceinline__ double tan_y(const TanCols& t, int j) {
+    return j == 2 ? 1.0 + t.c[2].y : j == 3 ? t.s + t.c[3].y : t.c[j].y;
+}
 
 template <bool DEC>
 __device__ __forceinline__ constexpr bool tan_has_x(int j) { return !DEC || j < 2 || j > 3; }
@@ -122,6 +134,9 @@ __device__ __forceinline__ void tan_drift(const P6& r, TanCols& t, const DriftIn
             c.ct = fma(ty, c.py, c.ct);
         }
     }
+    t.s += n;
+    t.sx += tx;
+    t.sy += ty;
     TanCol& e = t.c[4];
     const double fe = f * pe;
     e.x = fma(-fe, d.x, e.x);
@@ -142,14 +157,15 @@ __device__ __forceinline__ void tan_kick(const P6& r, TanCols& t, const PL& pl, 
 #pragma unroll
     for (int j = 0; j < (HASK ? 6 : 5); ++j) {
         TanCol& c = t.c[j];
+        const double x = tan_x(t, j), y = tan_y(t, j);
         if (tan_has_x<DEC>(j)) {
-            c.px = fma(-ax, c.x, c.px);
-            if (BEND) c.ct = fma(lirho, c.x, c.ct);
+            c.px = fma(-ax, x, c.px);
+            if (BEND) c.ct = fma(lirho, x, c.ct);
         }
-        if (tan_has_y<DEC>(j)) c.py = fma(ay, c.y, c.py);
+        if (tan_has_y<DEC>(j)) c.py = fma(ay, y, c.py);
         if (!DEC) {
-            c.px = fma(b, c.y, c.px);
-            c.py = fma(b, c.x, c.py);
+            c.px = fma(b, y, c.px);
+            c.py = fma(b, x, c.py);
         }
     }
     if (BEND) t.c[4].px += li;
@@ -359,9 +375,9 @@ __device__ __forceinline__ void tan_drift6(P6& r, const TanMap& J, double L, dou
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
         const double dpx = J.at(1, j), dpy = J.at(3, j), dd = J.at(4, j);
-        J.at(0, j) = fma(nl, dpx, fma(-tx, dd, J.at(0, j)));
-        J.at(2, j) = fma(nl, dpy, fma(-ty, dd, J.at(2, j)));
-        J.at(5, j) = fma(tx, dpx, fma(ty, dpy, fma(tc, dd, J.at(5, j))));
+        J.at(0, j) += fma(nl, dpx, -(tx * dd));
+        J.at(2, j) += fma(nl, dpy, -(ty * dd));
+        J.at(5, j) += fma(tx, dpx, fma(ty, dpy, tc * dd));
     }
     drift6_pn<false>(r, L, pn);
 }
@@ -393,7 +409,7 @@ __device__ __forceinline__ void tan_magnet(P6& r, Recip& rc, const TanMap& J, co
     TanCols t;
 #pragma unroll
     for (int j = 0; j < 6; ++j) t.c[j] = TanCol{0.0, 0.0, 0.0, 0.0, 0.0};
-    t.c[0].x = t.c[1].px = t.c[2].y = t.c[3].py = 1.0;
+    t.s = t.sx = t.sy = 0.0;
     double irho = 0.0;
     if (BEND) {
         irho = e.f(ATB_BM_IRHO);
@@ -425,8 +441,8 @@ __device__ __forceinline__ void tan_magnet(P6& r, Recip& rc, const TanMap& J, co
         const double fx = e.f(ATB_BM_FXOUT);
 #pragma unroll
         for (int j = 0; j < (HASK ? 6 : 5); ++j) {
-            t.c[j].px = fma(fx, t.c[j].x, t.c[j].px);
-            t.c[j].py = fma(-fy, t.c[j].y, t.c[j].py);
+            t.c[j].px = fma(fx, tan_x(t, j), t.c[j].px);
+            t.c[j].py = fma(-fy, tan_y(t, j), t.c[j].py);
         }
         t.c[4].py = fma(-r.y, dfy, t.c[4].py);
         edge_fringe<false>(r, irho, e.f(ATB_BM_EOUT), e.f(ATB_BM_FCOUT), e.f(ATB_BM_FXOUT),
@@ -439,9 +455,14 @@ __device__ __forceinline__ void tan_magnet(P6& r, Recip& rc, const TanMap& J, co
     /* J <- M J */
 #pragma unroll 2
     for (int j = 0; j < 6; ++j) {
-        double v[5], s[5] = {0.0, 0.0, 0.0, 0.0, J.at(5, j)};
+        double v[5], s[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) v[k] = J.at(k, j);
+        s[0] = t.s * v[1];
+        s[1] = 0.0;
+        s[2] = t.s * v[3];
+        s[3] = 0.0;
+        s[4] = fma(t.sx, v[1], t.sy * v[3]);
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
             s[0] = fma(t.c[k].x, v[k], s[0]);
@@ -450,8 +471,8 @@ __device__ __forceinline__ void tan_magnet(P6& r, Recip& rc, const TanMap& J, co
             s[3] = fma(t.c[k].py, v[k], s[3]);
             s[4] = fma(t.c[k].ct, v[k], s[4]);
         }
-        J.at(0, j) = s[0]; J.at(1, j) = s[1]; J.at(2, j) = s[2];
-        J.at(3, j) = s[3]; J.at(5, j) = s[4];
+        J.at(0, j) = v[0] + s[0]; J.at(1, j) = v[1] + s[1]; J.at(2, j) = v[2] + s[2];
+        J.at(3, j) = v[3] + s[3]; J.at(5, j) += s[4];
     }
     if (mixed) tan_mix_exit(J, &mix);
     tan_exit(r, J, e, HASK ? g : nullptr);
