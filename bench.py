@@ -12,8 +12,9 @@ Arms:
                      launching stream, L2 flushed between steps) with the
                      particles resident in HBM; ``e2e``: the drop-in call
                      ``at_b200.gpupass`` on pinned host arrays (host->device
-                     and device->host copies of the bunch and loss map inside
-                     the timed region).
+                     and device->host copies of the bunch and of the loss
+                     flags inside the timed region, and of the rest of the
+                     loss map in the steps that lose particles).
   --impl reference   the reference's own compiled C engine (pyat/at.c +
                      atintegrators, built by oracle/build_ref.py) through its
                      atpass entry, OpenMP over all host cores, on a bounded
@@ -443,21 +444,22 @@ def run_b200(a):
         line = list(ring)
         line_obj = type(ring)(line, energy=ring.energy, particle=ring.particle)
         tracking.gpupass(line_obj, rh, 1, losses=True, mode=mode, gpu_pool=[local])
-        etimes = []
+        etimes, d2h = [], 0
         if world > 1:
             dist.barrier()
         for k in range(a.steps):
             torch.cuda.synchronize()
             t0 = time.perf_counter()
-            tracking.gpupass(line_obj, rh, T, losses=True, reuse=True, keep_counter=True,
-                             mode=mode, gpu_pool=[local])
+            _, ld = tracking.gpupass(line_obj, rh, T, losses=True, reuse=True, keep_counter=True,
+                                     mode=mode, gpu_pool=[local])
             etimes.append(time.perf_counter() - t0)
+            d2h += d2h_bytes(N, ld)
         et = torch.tensor([sum(etimes)], dtype=torch.float64, device=dev)
         if world > 1:
             dist.all_reduce(et, op=dist.ReduceOp.MAX)
         e2e = {"value": world * N * T * a.steps / float(et.item()), "unit": UNIT,
                "h2d_bytes_per_step": N * 48,
-               "d2h_bytes_per_step": N * 48 + N * (1 + 4 + 4 + 48),
+               "d2h_bytes_per_step": d2h // max(a.steps, 1),
                "api": "at_b200.gpupass (reference gpupass/atpass signature), pinned host arrays"}
 
     cpu = None
@@ -530,6 +532,13 @@ def run_b200(a):
     return 0
 
 
+def d2h_bytes(n, loss):
+    """Bytes that ``gpupass(..., losses=True)`` copies back for ``n``
+    particles: the coordinates and the loss flags, and where something was
+    lost the rest of the loss map (turn, element, coordinates)."""
+    return n * (48 + 1) + (n * (4 + 4 + 48) if loss["islost"].any() else 0)
+
+
 def _fodo_rates(device, mode, ring, r0, n, nt):
     import torch
 
@@ -572,7 +581,7 @@ def _fodo_rates(device, mode, ring, r0, n, nt):
         e2e.append(time.perf_counter() - t0)
     return {"value": n * nt / min(times), "unit": UNIT, "device_s": min(times),
             "e2e": {"value": n * nt / min(e2e[1:]), "unit": UNIT, "wall_s": min(e2e[1:]),
-                    "h2d_bytes": n * 48, "d2h_bytes": n * (48 + 57)},
+                    "h2d_bytes": n * 48, "d2h_bytes": d2h_bytes(n, ld)},
             "lost": int(ld["islost"].sum()), "arithmetic": mode}
 
 
