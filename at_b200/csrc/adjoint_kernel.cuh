@@ -47,7 +47,7 @@
  * Bound by dependent FP64 latency at 3.5 warps a scheduler (65,536 particles).
  * A turn of the FODO ring with 128 strengths backwards: 5.0 ms with the step
  * entries recomputed into shared memory and every step run twice more; 2.3 ms
- * with the stages undone from the exit (0.9 of it the tracking), which needs
+ * with the stages undone from the exit (0.8 of it the tracking), which needs
  * no store and keeps one stage's coordinates instead of seven.
  */
 #ifndef ATB_ADJOINT_KERNEL_CUH

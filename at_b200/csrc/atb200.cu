@@ -423,10 +423,10 @@ int launch(atb_handle* h, const std::vector<AtbJob>& jobs, const std::vector<Atb
    (to a multiple of 32) when the set does not fill every SM with full blocks,
    so that a few hundred particles run on many SMs rather than queue on a few,
    and a set between one and two blocks an SM takes two equal ones (50,000
-   particles x 1 turn of the large ring 10.3 -> 8.5 ms: 12 warps on every SM
+   particles x 1 turn of the large ring 8.9 -> 7.6 ms: 12 warps on every SM
    instead of 16 on some).  Beyond two blocks an SM, equal shares of what is
-   left after the full waves are slower than full blocks on some SMs: 100,003
-   particles there 16.8 against 15.4 ms.  Results do not depend on it:
+   left after the full waves were slower than full blocks on some SMs (100,003
+   particles there by 9 %).  Results do not depend on it:
    particles are independent. */
 int threads_for(const atb_handle* h, int64_t np) {
     const int64_t sms = std::max(h->sm_count, 1), full = h->threads;
@@ -924,10 +924,10 @@ int atb_track(atb_handle* h, int32_t id, double* rin, int64_t np, int32_t nturns
     int64_t turns_per_chunk = nturns;
     if (nref > 0 && rec_turn > 0)
         turns_per_chunk = std::max<int64_t>(1, h->rout_budget / (rec_turn * slot_bytes));
-    /* Snapshots of some size come back while the next turns are tracked: at
-       least four chunks of turns, none larger than a staging buffer, each in
-       its own part of the device buffer (10,007 particles x 10 turns of the
-       FODO ring with 32 points, 154 MB: 12.8 -> 9.3 ms). */
+    /* Snapshots of some size come back while the next turns are tracked: a
+       quarter of the turns a chunk (rounded up), no chunk larger than a staging
+       buffer, each in its own part of the device buffer (10,007 particles x 10
+       turns of the FODO ring with 32 points, 154 MB: 12.8 -> 9.3 ms). */
     const int64_t turn_bytes = rec_max * slot_bytes;
     const bool piped = nref > 0 && group == np && nturns > 1 && turns_per_chunk >= nturns &&
                        turn_bytes > 0 && turn_bytes <= kStageBytes &&

@@ -86,10 +86,6 @@ ATB_RN_FN bool rn_within(double v, uint32_t lo_hi, uint32_t hi_hi) {
 ATB_RN_FN bool rn_below(double v, uint32_t hi_hi) {
     return (rn_hi(v) & 0x7fffffffu) < hi_hi;
 }
-/* 1 - 2^-53, the all-ones significand next to one */
-ATB_RN_FN bool rn_below_one(double v) {
-    return rn_hi(v) == 0x3fefffffu && rn_lo(v) == 0xffffffffu;
-}
 /* 1 + delta in a magnet without radiation, in [1/2, 2) */
 ATB_RN_FN bool rn_opd_constant(double o) { return rn_within(o, 0x3fe00000u, 0x40000000u); }
 /* 1 + delta at the entry of a radiating magnet, in [97/128, 5/4): the kicks
@@ -97,16 +93,10 @@ ATB_RN_FN bool rn_opd_constant(double o) { return rn_within(o, 0x3fe00000u, 0x40
    2^-14) leave it in (0.7072, 1.4141), where its square and that of its
    reciprocal are between 1/2 and 2 */
 ATB_RN_FN bool rn_opd_fits(double o) { return rn_within(o, 0x3fe84000u, 0x3ff40000u); }
-/* divisors of rn_rcp_near: normal, below 2^1000 */
-ATB_RN_FN bool rn_near_fits(double d) { return rn_within(d, 0x00100000u, 0x7e700000u); }
-/* the same of divisors known to be at least 1 */
-ATB_RN_FN bool rn_nearer_fits(double d) { return rn_within(d, 0x3ff00000u, 0x7e700000u); }
 /* What is left to exclude per particle are tiny nonzero values, whose
    remainders or squares would underflow: two integer instructions each, zeros
    passing.  A denormal below 2^-1042 has a zero high word and passes as well;
    rn_denormal finds it where it would matter. */
-/* v >= 0: zero or at least 2^-860 */
-ATB_RN_FN bool rn_square_fits(double v) { return rn_hi(v) - 1u >= 0x0a300000u - 1u; }
 /* |v| zero or at least 2^-480 */
 ATB_RN_FN bool rn_not_tiny(double v) {
     const uint32_t h = rn_hi(v);
@@ -129,6 +119,19 @@ ATB_RN_FN bool rn_denormal(double v) { return 2u * rn_hi(v) == 0u && rn_lo(v) !=
 ATB_RN_FN bool rn_ordinary(double v) {
     return rn_not_tiny(v) && !rn_denormal(v) && rn_below(v, 0x58f00000u);
 }
+
+/* The domains of single operations, for the tests: the kernels need no test of
+   their own for them. */
+/* 1 - 2^-53, the all-ones significand next to one */
+ATB_RN_FN bool rn_below_one(double v) {
+    return rn_hi(v) == 0x3fefffffu && rn_lo(v) == 0xffffffffu;
+}
+/* divisors of rn_rcp_near: normal, below 2^1000 */
+ATB_RN_FN bool rn_near_fits(double d) { return rn_within(d, 0x00100000u, 0x7e700000u); }
+/* the same of divisors known to be at least 1 */
+ATB_RN_FN bool rn_nearer_fits(double d) { return rn_within(d, 0x3ff00000u, 0x7e700000u); }
+/* v >= 0: zero or at least 2^-860 */
+ATB_RN_FN bool rn_square_fits(double v) { return rn_hi(v) - 1u >= 0x0a300000u - 1u; }
 
 /* ---- arithmetic --------------------------------------------------------- */
 

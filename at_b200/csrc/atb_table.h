@@ -179,7 +179,7 @@
  * (tangent_plain.cuh) covers an element: everything but radiating magnets,
  * field scaling, quadrupole fringes, bend edges of method 3, thick correctors
  * and other integrators.  A lattice takes that kernel when all its elements
- * do (the FODO ring's turn of 65,536 particles 3.72 ms), else the one on dual
+ * do (the FODO ring's turn of 65,536 particles 3.83 ms), else the one on dual
  * numbers (12.9 ms there). */
 static inline int atb_tangent_by_hand(unsigned op, unsigned fl) {
     if (op == ATB_OP_STRMPOLE_RAD || op == ATB_OP_BNDMPOLE_RAD) return 0;

@@ -11,14 +11,14 @@
  * and ct need no column of their own (delta is constant, ct feeds nothing),
  * and in upright magnets up to the quadrupole the planes do not mix.  The
  * tangent map J(s) = d r(s) / d r0 of the particle waits in shared memory and
- * is multiplied by the magnet's matrix once per magnet.
+ * is updated by the magnet's matrix once per magnet.
  *
  * Bound: the FP64 pipe when the SMs are full, dependent latency below that
  * (one warp a scheduler up to 19,000 particles).  One turn of the FODO ring with
- * 128 strengths: 16,411 particles 1.50 ms (4.6 on dual numbers), 65,536
- * particles 3.72 ms (12.9).  168 registers and three blocks an SM: with 128
+ * 128 strengths: 16,411 particles 1.58 ms (4.6 on dual numbers), 65,536
+ * particles 3.83 ms (12.9).  168 registers and three blocks an SM: with 128
  * and four the columns spill (3 KB of stores), with 255 and two the larger set
- * takes 3.85 ms.
+ * takes 3 % longer.
  */
 #ifndef ATB_TANGENT_PLAIN_CUH
 #define ATB_TANGENT_PLAIN_CUH

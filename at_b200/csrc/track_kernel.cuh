@@ -167,7 +167,7 @@ __device__ __forceinline__ void misalign_rotation(P6T<T>& r, const double* m, bo
 /* The usual misalignment, a shift and a rotation of the x/y planes: one branch,
  * and the fourteen words (16-byte aligned blocks) asked for at once.  One by
  * one, each branch waited for its own words: 375 cycles a warp and magnet with
- * 16 warps on an SM, 172 so. */
+ * 16 warps on an SM, 208 so. */
 struct ShiftTilt {
     double2 t[3], m[4];
 };
@@ -450,8 +450,8 @@ __device__ __noinline__ P6 multipole_steps_call(P6 r, Rec e, Param pm, double nl
  * of atb_rn.h: the same IEEE results, straight-line code in the step loop.
  * The divisions bounded these loops: about nine FP64 instructions each, a
  * seed on the XU pipe and a branch to a slow path that ended the block the
- * compiler could interleave (a plain sextupole step of a lone warp took 631
- * cycles and takes 275, of 16 warps a scheduler 296 and 160).  The last drift
+ * compiler could interleave (a sextupole step without radiation took a lone
+ * warp 631 cycles and takes 271, one with radiation 1,886 and 724).  The last drift
  * of a step and the first of the next have the same length, momenta and
  * 1/(1+delta), hence the same increments: they are computed once and added
  * twice.
@@ -1005,7 +1005,7 @@ __device__ __forceinline__ void track_integ(P6& r, Recip& c, const Rec& e, const
  * arithmetic on x and y.  With cavities, fringes and the rest beside them the
  * particle moved between registers around every element (159 instructions for
  * a drift, 14 of them FP64, where it now takes 88; a quadrupole beside its
- * steps 1,060 cycles of a lone warp instead of 1,400).  A call that takes and
+ * steps 1,020 cycles of a lone warp instead of 1,400).  A call that takes and
  * returns the whole particle costs some 600 cycles: with it a marker took 1,400,
  * now 720, a thin multipole 2,000, now 1,200, a drift with apertures 2,300, now
  * 1,700. */
